@@ -36,13 +36,19 @@
 namespace gbc {
 namespace {
 
-constexpr int CT = 128;     // threads per block
-constexpr int SITES = 32;   // sites per block -> 96 rows (site, colour)
+constexpr int SITES = 32;          // sites per block, one per lane -> 96 rows (site, colour)
 constexpr int ROWS = SITES * 3;
-constexpr int DP = ROWS + 8;  // pitch of the transposed delta tile: 52 words = 4 mod 8 (conflict-free)
+constexpr int DIRS = 9;            // the site itself and 8 hops, one warp each
+constexpr int CT = 32 * DIRS;      // threads per block
+
+enum { IN_ODD = 1, OUT_ODD = 2 };  // layer input zero on the even sites; output wanted on the odd sites only
 
 __host__ __device__ constexpr int kpad(int cin) { return ((9 * cin * 2 + 15) / 16) * 16; }
 __host__ __device__ constexpr int npad(int cout) { return ((2 * cout + 7) / 8) * 8; }
+
+// The GEMM's K index is (d * CIN + i) * 2 + re/im.  Its N index is comp(o, re/im), the order of the
+// activation planes, (re_o, re_o+1, im_o, im_o+1) for even o, so an accumulator row is stored as it is.
+__host__ __device__ constexpr int comp(int i, int im) { return (i >> 1) * 4 + 2 * im + (i & 1); }
 
 __device__ __forceinline__ uint32_t bf16x2(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -53,171 +59,99 @@ __device__ __forceinline__ Coord eo_coords(const Geom& g, int j) {
   const int par = j >= g.Vh ? 1 : 0;
   return cb_coords(g, j - par * g.Vh, par);
 }
-__device__ __forceinline__ int eo_index(const Geom& g, const Coord& c) {
-  const int par = (c.x[0] + c.x[1] + c.x[2] + c.x[3]) & 1;
-  return par * g.Vh + cb_index(g, c);
+
+// Activations are planes of float4 over the even-odd site index: plane a * C/2 + i/2 holds
+// (re, re, im, im) of channels i, i + 1 and colour a, so the 32 lanes of a warp (32 consecutive
+// sites) read and write 512 contiguous bytes per plane.
+__host__ __device__ constexpr int planes(int ch) { return 3 * ch / 2; }
+
+// Byte offset of the 16-byte core-matrix row (row, 8-element column chunk) of a staged bf16 tile of
+// COLS columns: the tensor cores' canonical K-major layout without swizzle, 8 x 8 core matrices
+// (8 rows of 16 bytes, 128 contiguous bytes), 128 bytes apart along the columns (the descriptor's
+// leading byte offset), row groups COLS * 16 bytes apart (its stride byte offset).  Rows are
+// colour * 32 + site, so the 8 lanes of a quarter warp fill one core matrix: no bank conflicts.
+template <int COLS>
+__device__ __forceinline__ uint32_t core_row(int row, int chunk) {
+  return (uint32_t)((row >> 3) * (COLS * 16) + chunk * 128 + (row & 7) * 16);
 }
 
-// Row pitch (bf16 elements) of the staged tiles: at least kpad(cin), with the pitch in 32-bit words
-// = 4 mod 8, so that the 8 rows x 4 column pairs an mma fragment load touches fall in 32 distinct
-// shared-memory banks (a pitch of 224 elements put them on 8 banks: 4-way conflicts).
-__host__ __device__ constexpr int gpitch(int cin) {
-  return kpad(cin) + ((4 - (kpad(cin) / 2) % 8 + 8) % 8) * 2;
-}
-
-// Where element (row, k) of a staged bf16 tile lives, in elements from the tile base:
-//  - PitchLayout: row-major at pitch gpitch(cin) (the mma.sync fragments of the weight gradient);
-//  - CoreLayout: the tensor cores' canonical K-major layout without swizzle, read by tcgen05.mma
-//    through a shared-memory descriptor: 8 x 8 core matrices (8 rows of 16 bytes, 128 contiguous
-//    bytes), the core matrices of a row group along K 128 bytes apart (the descriptor's leading
-//    byte offset), row groups KP * 16 bytes apart (its stride byte offset).
-template <int CIN>
-struct PitchLayout {
-  __device__ __forceinline__ int operator()(int row, int k) const { return row * gpitch(CIN) + k; }
-};
-template <int CIN>
-struct CoreLayout {
-  __device__ __forceinline__ int operator()(int row, int k) const {
-    return (row >> 3) * (kpad(CIN) * 8) + (k >> 3) * 64 + (row & 7) * 8 + (k & 7);
-  }
-};
-
-// the 9 sites each site of the tile reads (d = 0 itself, 1 + 2 mu forward, 2 + 2 mu backward)
-__device__ void tile_neighbours(int (*nbr)[9], const Geom& g, int V, int site0) {
-  for (int p = threadIdx.x; p < SITES * 9; p += blockDim.x) {
-    const int s = p / 9, d = p % 9, j = site0 + s;
-    int n = j;
-    if (j < V && d > 0) {
-      Coord c = eo_coords(g, j);
-      const int mu = (d - 1) >> 1;
-      if (((d - 1) & 1) == 0) c.x[mu] = c.x[mu] + 1 == g.L[mu] ? 0 : c.x[mu] + 1;
-      else c.x[mu] = c.x[mu] == 0 ? g.L[mu] - 1 : c.x[mu] - 1;
-      n = eo_index(g, c);
-    }
-    nbr[s][d] = n;
-  }
-}
-
-// G[row = s*3 + a][k = (d*CIN + i)*2 + re/im] = (T_d h)(site)[i][a] in BF16, row pitch GP; the K
-// padding zeroed.  One task per (site, direction, channel), channel fastest: consecutive threads
-// read consecutive channel vectors and write consecutive 32-bit words (re, im packed), and the
-// link of a (site, direction) is shared through L1 by the threads of its channels.
-template <int CIN, class Lay>
-__device__ void gather_tile(__nv_bfloat16* G, const int (*nbr)[9], int V, const float2* links, const float2* h,
-                            int site0, Lay lay) {
-  for (int p = threadIdx.x; p < SITES * 9 * CIN; p += blockDim.x) {
-    const int i = p % CIN, sd = p / CIN, s = sd % SITES, d = sd / SITES;
-    const int j = site0 + s;
-    const int k = (d * CIN + i) * 2;
-    auto put = [&](int a, uint32_t v) { *reinterpret_cast<uint32_t*>(G + lay(s * 3 + a, k)) = v; };
-    if (j >= V) {
-      put(0, 0u);
-      put(1, 0u);
-      put(2, 0u);
-      continue;
-    }
-    const int n = nbr[s][d];
-    const float2* src = h + ((size_t)n * CIN + i) * 3;
-    const float2 x0 = src[0], x1 = src[1], x2 = src[2];
-    if (d == 0) {
-      put(0, bf16x2(x0.x, x0.y));
-      put(1, bf16x2(x1.x, x1.y));
-      put(2, bf16x2(x2.x, x2.y));
-      continue;
-    }
-    const int mu = (d - 1) >> 1;
-    const bool bwd = ((d - 1) & 1) != 0;
-    // T_{+mu} h = U_mu(x) h(x+mu);  T_{-mu} h = U_mu(x-mu)^dag h(x-mu)
-    const float2* L = links + ((size_t)(bwd ? n : j) * 4 + mu) * 9;
+// The neighbour that direction d of site i (parity par) reads, as an even-odd index
+__device__ __forceinline__ int neighbour(const Geom& g, int par, int i, int d) {
+  if (d == 0) return par * g.Vh + i;
+  Coord c = cb_coords(g, i, par);
+  const int mu = (d - 1) >> 1;
+  const bool bwd = ((d - 1) & 1) != 0;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      float2 u0, u1, u2;
-      if (!bwd) {
-        u0 = L[3 * a];
-        u1 = L[3 * a + 1];
-        u2 = L[3 * a + 2];
-      } else {
-        u0 = make_float2(L[a].x, -L[a].y);
-        u1 = make_float2(L[3 + a].x, -L[3 + a].y);
-        u2 = make_float2(L[6 + a].x, -L[6 + a].y);
+  for (int m = 0; m < 4; ++m)
+    if (m == mu) c.x[m] = bwd ? (c.x[m] == 0 ? g.L[m] - 1 : c.x[m] - 1) : (c.x[m] + 1 == g.L[m] ? 0 : c.x[m] + 1);
+  return (1 - par) * g.Vh + cb_index(g, c);
+}
+
+// M_d of a site: U_mu(x) for +mu, U_mu(x - mu)^dag for -mu; links are planes [mu * 9 + entry][V]
+__device__ __forceinline__ void load_transport(float2 (&m)[9], const float2* links, int V, int j, int n, int d) {
+  const int mu = (d - 1) >> 1;
+  if ((d - 1) & 1) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const float2 u = __ldg(links + (size_t)(mu * 9 + 3 * k + a) * V + n);
+        m[3 * a + k] = make_float2(u.x, -u.y);
       }
-      const float re = u0.x * x0.x - u0.y * x0.y + u1.x * x1.x - u1.y * x1.y + u2.x * x2.x - u2.y * x2.y;
-      const float im = u0.x * x0.y + u0.y * x0.x + u1.x * x1.y + u1.y * x1.x + u2.x * x2.y + u2.y * x2.x;
-      put(a, bf16x2(re, im));
-    }
-  }
-  // zero the K padding
-  constexpr int K = 9 * CIN * 2, KP = kpad(CIN);
-  if (KP > K)
-    for (int p = threadIdx.x; p < ROWS * (KP - K); p += blockDim.x) {
-      const int r = p / (KP - K), k = K + p % (KP - K);
-      G[lay(r, k)] = __float2bfloat16(0.f);
-    }
-}
-
-// The block's transports staged once: lk[s][d - 1][3 a + k] = M_d[a][k] with M_{+mu} = U_mu(x) and
-// M_{-mu} = U_mu(x - mu)^dag, for every direction d = 1..8 of the SITES sites.  The forward layer
-// reads them for every right-hand side of the batch instead of reloading the link per channel.
-__device__ void stage_transports(float2 (*lk)[8][9], const int (*nbr)[9], int V, const float2* links, int site0) {
-  for (int p = threadIdx.x; p < SITES * 8 * 9; p += blockDim.x) {
-    const int e = p % 9, sd = p / 9, s = sd / 8, d = sd % 8 + 1;
-    const int j = site0 + s;
-    if (j >= V) continue;
-    const int mu = (d - 1) >> 1;
-    const bool bwd = ((d - 1) & 1) != 0;
-    const int a = e / 3, k = e % 3;
-    const float2* L = links + ((size_t)(bwd ? nbr[s][d] : j) * 4 + mu) * 9;
-    const float2 u = bwd ? L[3 * k + a] : L[3 * a + k];
-    lk[s][d - 1][e] = bwd ? make_float2(u.x, -u.y) : u;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 9; ++e) m[e] = __ldg(links + (size_t)(mu * 9 + e) * V + j);
   }
 }
 
-// G as gather_tile, from staged transports: one task per (site, direction, channel), channel
-// fastest, so that consecutive threads read consecutive channel vectors of a neighbour and write
-// consecutive words of a row; the transport comes from shared memory instead of the links.
-template <int CIN, class Lay>
-__device__ void gather_tile_staged(__nv_bfloat16* G, const int (*nbr)[9], const float2 (*lk)[8][9], int V,
-                                   const float2* h, int site0, Lay lay) {
-  for (int p = threadIdx.x; p < SITES * 9 * CIN; p += blockDim.x) {
-    const int i = p % CIN, sd = p / CIN, s = sd % SITES, d = sd / SITES;
-    const int j = site0 + s;
-    const int k = (d * CIN + i) * 2;
-    auto put = [&](int a, uint32_t v) { *reinterpret_cast<uint32_t*>(G + lay(s * 3 + a, k)) = v; };
-    if (j >= V) {
-      put(0, 0u);
-      put(1, 0u);
-      put(2, 0u);
-      continue;
-    }
-    const float2* src = h + ((size_t)nbr[s][d] * CIN + i) * 3;
-    const float2 x0 = src[0], x1 = src[1], x2 = src[2];
+// One component of M x in FP32, (re, im) rounded to BF16.  The FMA order is spelled out: a last-bit
+// change here flips BF16 roundings, which the following layers carry on.
+__device__ __forceinline__ uint32_t transported(float2 u0, float2 u1, float2 u2, float x0r, float x0i, float x1r,
+                                                float x1i, float x2r, float x2i) {
+  float re = __fmaf_rn(u0.x, x0r, -__fmul_rn(u0.y, x0i));
+  float im = __fmaf_rn(u0.x, x0i, __fmul_rn(u0.y, x0r));
+  re = __fmaf_rn(-u1.y, x1i, __fmaf_rn(u1.x, x1r, re));
+  im = __fmaf_rn(u1.y, x1r, __fmaf_rn(u1.x, x1i, im));
+  re = __fmaf_rn(-u2.y, x2i, __fmaf_rn(u2.x, x2r, re));
+  im = __fmaf_rn(u2.y, x2r, __fmaf_rn(u2.x, x2i, im));
+  return bf16x2(re, im);
+}
+
+// One (site, direction) of the gathered tile: the channels of site n in chunks of four, transported
+// by m (d > 0), rounded to BF16 and written as one 16-byte core-matrix row per colour and chunk.
+// The transport stays in registers for all channels (and, in the callers, all right-hand sides).
+template <int CIN>
+__device__ __forceinline__ void gather_dir(unsigned char* G, int d, int s, const float2 (&m)[9], const float4* h,
+                                           int V, int n) {
+#pragma unroll
+  for (int c = 0; c < CIN / 4; ++c) {
+    float4 x[3][2];
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) x[k][q] = __ldg(h + (size_t)(k * (CIN / 2) + 2 * c + q) * V + n);
+    const int chunk = d * (CIN / 4) + c;
     if (d == 0) {
-      put(0, bf16x2(x0.x, x0.y));
-      put(1, bf16x2(x1.x, x1.y));
-      put(2, bf16x2(x2.x, x2.y));
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        *reinterpret_cast<uint4*>(G + core_row<kpad(CIN)>(a * 32 + s, chunk)) =
+            make_uint4(bf16x2(x[a][0].x, x[a][0].z), bf16x2(x[a][0].y, x[a][0].w), bf16x2(x[a][1].x, x[a][1].z),
+                       bf16x2(x[a][1].y, x[a][1].w));
       continue;
     }
-    const float2* m = lk[s][d - 1];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       const float2 u0 = m[3 * a], u1 = m[3 * a + 1], u2 = m[3 * a + 2];
-      const float re = u0.x * x0.x - u0.y * x0.y + u1.x * x1.x - u1.y * x1.y + u2.x * x2.x - u2.y * x2.y;
-      const float im = u0.x * x0.y + u0.y * x0.x + u1.x * x1.y + u1.y * x1.x + u2.x * x2.y + u2.y * x2.x;
-      put(a, bf16x2(re, im));
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const float4 x0 = x[0][q], x1 = x[1][q], x2 = x[2][q];
+        w[2 * q] = transported(u0, u1, u2, x0.x, x0.z, x1.x, x1.z, x2.x, x2.z);
+        w[2 * q + 1] = transported(u0, u1, u2, x0.y, x0.w, x1.y, x1.w, x2.y, x2.w);
+      }
+      *reinterpret_cast<uint4*>(G + core_row<kpad(CIN)>(a * 32 + s, chunk)) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
-  // zero the K padding
-  constexpr int K = 9 * CIN * 2, KP = kpad(CIN);
-  if (KP > K)
-    for (int p = threadIdx.x; p < ROWS * (KP - K); p += blockDim.x) {
-      const int r = p / (KP - K), k = K + p % (KP - K);
-      G[lay(r, k)] = __float2bfloat16(0.f);
-    }
-}
-
-__device__ __forceinline__ uint32_t ld_bf16x2(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
-__device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-  return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
@@ -292,31 +226,39 @@ __device__ __forceinline__ void tmem_load_row(uint32_t taddr, float (&v)[NU]) {
 __host__ __device__ constexpr int nump(int cout) { return ((2 * cout + 15) / 16) * 16; }  // N of the MMA
 constexpr int kTmemCols = 32;  // tensor-memory columns allocated per block (>= nump, power of 2)
 
-// out[b][j][o][a] = (G W^T)[row][2o + re/im] for every right-hand side b of the batch: the
-// weights and (for batches) the block's transports are staged once, then per b the gathered tile G
-// and its GEMM on the tensor cores
+// out[b] = (G W^T) for the right-hand sides b of this block: warp d gathers direction d of the
+// block's 32 sites (all of one parity; lane = site) into the BF16 tile G, one thread issues the
+// GEMM on the tensor cores, and warps 0..2 write colours 0..2 from their accumulator lanes.
+// What bounds it: the gather's loads through L1/L2 (9 neighbours x C_in x 24 B per site and
+// right-hand side).  Against one task per (site, direction, channel) with the transports in shared
+// memory, this mapping reads whole 512-byte rows, keeps each transport in registers for every
+// channel and right-hand side and writes 16 bytes per shared-memory store.  A 12 -> 12 layer at
+// 16^3 x 32: 1772 -> 492 us for 12 right-hand sides, 217 -> 60 us for one (kernel time, cold L2).
+// IN_ODD: only the self term of odd sites and the hops of even sites are non-zero; the others'
+// columns of G are zeroed once, and odd sites need only the K steps that cover the self term.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT) layer_kernel(Geom g, int V, int batch, const float2* links, const float2* hin,
-                                                   float2* hout, const __nv_bfloat16* Wr) {
+__global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int batch, int per, int flags,
+                                                      const float2* __restrict__ links, const float4* __restrict__ hin,
+                                                      float4* __restrict__ hout, const uint4* __restrict__ Wc) {
   constexpr int KP = kpad(CIN), NP = npad(COUT), NU = nump(COUT);
   constexpr int MROWS = 128;  // the MMA's M: the 96 rows of the tile and 32 discarded rows
   static_assert(ROWS <= MROWS && NU <= kTmemCols, "tile does not fit the MMA");
+  // G (96 rows), then W (NP rows); the MMA's rows 96..127 and weight rows NP..NU-1 read what
+  // follows, inside the launch's 128 rows: their results are never read back
   extern __shared__ __align__(128) unsigned char smem[];
-  // G holds the tile's 96 rows; the MMA's rows 96..127 read whatever follows (the weights, the
-  // staged transports or the padding the launch adds): their results are never read back
-  // (likewise the MMA's weight rows NP..NU-1, whose result columns are never read back)
-  __nv_bfloat16* G = reinterpret_cast<__nv_bfloat16*>(smem);  // CoreLayout, ROWS x KP
-  __nv_bfloat16* W = G + ROWS * KP;                           // CoreLayout, NP x KP
-  float2(*lk)[8][9] = reinterpret_cast<float2(*)[8][9]>(W + NP * KP);
-  __shared__ int nbr[SITES][9];
+  unsigned char* G = smem;
+  unsigned char* W = smem + ROWS * KP * 2;
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
-  __shared__ int s_ok;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int site0 = blockIdx.x * SITES;
-  const CoreLayout<CIN> lay{};
-  for (int p = tid; p < NP * KP; p += blockDim.x) W[lay(p / KP, p % KP)] = Wr[p];
-  if (warp == 0) {
+  const int tid = threadIdx.x, d = tid >> 5, s = tid & 31;
+  int tile = blockIdx.x, par = 1;
+  if (!(flags & OUT_ODD)) {
+    par = tile >= tiles ? 1 : 0;
+    tile -= par * tiles;
+  }
+  const int b0 = blockIdx.y * per, b1 = min(batch, b0 + per);
+  for (int p = tid; p < NP * KP / 8; p += CT) reinterpret_cast<uint4*>(W)[p] = __ldg(Wc + p);
+  if (d == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_base)),
                  "r"(kTmemCols));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
@@ -326,29 +268,42 @@ __global__ void __launch_bounds__(CT) layer_kernel(Geom g, int V, int batch, con
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  tile_neighbours(nbr, g, V, site0);
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const uint32_t tmem = tmem_base;
-  // one right-hand side reads each transport once: it gathers straight from the links (the staged
-  // copy only costs shared memory and occupancy there)
-  const bool staged = batch > 1;
-  if (staged) stage_transports(lk, nbr, V, links, site0);
+  const int i = tile * SITES + s;
+  const bool valid = i < g.Vh;
+  const int ic = valid ? i : g.Vh - 1;  // lanes past the end gather the last site, store nothing
+  const int j = par * g.Vh + ic;
+  const bool mine = !(flags & IN_ODD) || ((d == 0) == (par == 1));
+  const int n = neighbour(g, par, ic, d);
+  float2 m[9];
+  if (mine && d > 0) load_transport(m, links, V, j, n, d);
+  constexpr int CH = CIN / 4;  // 16-byte chunks of a direction
+  if (!mine) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+#pragma unroll
+      for (int a = 0; a < 3; ++a)
+        *reinterpret_cast<uint4*>(G + core_row<KP>(a * 32 + s, d * CH + c)) = make_uint4(0, 0, 0, 0);
+  }
+  if (KP > 18 * CIN && d == 0) {
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      *reinterpret_cast<uint4*>(G + core_row<KP>(a * 32 + s, DIRS * CH)) = make_uint4(0, 0, 0, 0);
+  }
+  const int ksteps = (flags & IN_ODD) && par == 1 ? (2 * CIN + 15) / 16 : KP / 16;
   const uint64_t adesc = umma_desc(smem_u32(G), 128, KP * 16);
   const uint64_t bdesc = umma_desc(smem_u32(W), 128, KP * 16);
   constexpr uint32_t idesc = umma_idesc_bf16(MROWS, NU);
   bool ok = true;
-  for (int b = 0; b < batch && ok; ++b) {
-    __syncthreads();  // transports staged; the previous right-hand side's accumulators are read
-    if (staged) gather_tile_staged<CIN>(G, nbr, lk, V, hin + (size_t)b * V * CIN * 3, site0, lay);
-    else gather_tile<CIN>(G, nbr, V, links, hin + (size_t)b * V * CIN * 3, site0, lay);
-    // the tensor cores read G through the async proxy
+  for (int b = b0; b < b1; ++b) {
+    if (mine) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
+    // the tensor cores read G and W through the async proxy
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    __syncthreads();
+    // every thread leaves together once a wait for the previous right-hand side has given up
+    if (!__syncthreads_and(ok)) break;
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = tmem_base;
     if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-#pragma unroll
-      for (int ks = 0; ks < KP / 16; ++ks) {
+      for (int ks = 0; ks < ksteps; ++ks) {
         // K steps of 16 elements: two core matrices along K, 256 bytes
         const uint64_t da = adesc + (uint64_t)((ks * 256) >> 4), db = bdesc + (uint64_t)((ks * 256) >> 4);
         const uint32_t acc = ks > 0 ? 1u : 0u;
@@ -360,238 +315,344 @@ __global__ void __launch_bounds__(CT) layer_kernel(Geom g, int V, int batch, con
       asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                        smem_u32(&mbar))
                    : "memory");
-      s_ok = mbar_wait(smem_u32(&mbar), (uint32_t)(b & 1));
-      if (!s_ok) {
-        atomicAdd(&g_tc_wait_errors, 1);
-        // give the MMAs in flight one more bounded wait before their tensor memory is freed
-        (void)mbar_wait(smem_u32(&mbar), (uint32_t)(b & 1));
-      }
     }
-    __syncthreads();
-    ok = s_ok != 0;
-    if (!ok) break;
+    // every thread waits: the MMA has read G (the next gather may overwrite it) and written its
+    // accumulators
+    const uint32_t phase = (uint32_t)((b - b0) & 1);
+    ok = mbar_wait(smem_u32(&mbar), phase);
+    if (!ok) {
+      if (tid == 0) atomicAdd(&g_tc_wait_errors, 1);
+      // give the MMAs in flight one more bounded wait before their tensor memory is freed
+      (void)mbar_wait(smem_u32(&mbar), phase);
+      continue;
+    }
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const int row = warp * 32 + lane;
-    if (warp * 32 < ROWS) {  // warp 3 holds only padding rows
+    if (d < 3) {  // warp = colour, lane = site
       float v[NU];
-      tmem_load_row<NU>(tmem + ((uint32_t)(warp * 32) << 16), v);
-      const int s = row / 3, a = row % 3, j = site0 + s;
-      if (row < ROWS && j < V) {
-        float2* out = hout + (size_t)b * V * COUT * 3;
+      tmem_load_row<NU>(tmem + ((uint32_t)(d * 32) << 16), v);
+      if (valid) {
+        float4* out = hout + (size_t)b * V * planes(COUT) + j;
 #pragma unroll
-        for (int o = 0; o < COUT; ++o) out[((size_t)j * COUT + o) * 3 + a] = make_float2(v[2 * o], v[2 * o + 1]);
+        for (int q = 0; q < COUT / 2; ++q)
+          out[(size_t)(d * (COUT / 2) + q) * V] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
       }
+      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   }
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(kTmemCols));
+  if (d == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_base), "r"(kTmemCols));
 }
 
-// gradient of the real-form weights: dW[n][k] += sum_rows delta[row][n] * G[row][k]
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void ldmatrix2_trans(uint32_t (&r)[2], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];\n"
+               : "=r"(r[0]), "=r"(r[1])
+               : "r"(addr)
+               : "memory");
+}
+
+// Gradient of the real-form weights: dW[n][k] += sum_rows delta[row][n] G[row][k], a reduction over
+// every (site, colour, right-hand side).  Warp d gathers direction d of a 32-site tile as in
+// layer_kernel and multiplies exactly the K columns it gathered (no other warp reads them) by the
+// block's delta tile, both read through transposing ldmatrix from the core-matrix layout; the sums
+// stay in registers while the block walks its tiles, so each block adds to global memory once
+// (one atomic per weight and block instead of one per weight, tile and right-hand side, which took
+// most of the time: 769 -> 242 us for 12 -> 12 channels and 4 right-hand sides at 16^3 x 32).  The
+// delta tile is double buffered: one barrier per right-hand side.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT) wgrad_kernel(Geom g, int V, const float2* links, const float2* hin,
-                                                   const float2* delta, float* dW) {
-  constexpr int KP = kpad(CIN), NP = npad(COUT), MP = ((NP + 15) / 16) * 16, GP = gpitch(CIN);
-  extern __shared__ __align__(16) unsigned char smem[];
-  __nv_bfloat16* G = reinterpret_cast<__nv_bfloat16*>(smem);
-  __nv_bfloat16* Dt = G + ROWS * GP;  // [MP][DP]: delta transposed (A operand, row-major M x K)
-  __shared__ int nbr[SITES][9];
-  const int b = blockIdx.y;
-  const int site0 = blockIdx.x * SITES;
-  tile_neighbours(nbr, g, V, site0);
-  __syncthreads();
-  gather_tile<CIN>(G, nbr, V, links, hin + (size_t)b * V * CIN * 3, site0, PitchLayout<CIN>{});
-  const float2* dl = delta + (size_t)b * V * COUT * 3;
-  for (int p = threadIdx.x; p < MP * ROWS; p += blockDim.x) {
-    const int n = p / ROWS, row = p % ROWS;
-    const int s = row / 3, a = row % 3, j = site0 + s, o = n >> 1;
-    float v = 0.f;
-    if (n < 2 * COUT && j < V) {
-      const float2 d = dl[((size_t)j * COUT + o) * 3 + a];
-      v = (n & 1) ? d.y : d.x;
-    }
-    Dt[(size_t)n * DP + row] = __float2bfloat16(v);
+__global__ void __launch_bounds__(CT, 2) wgrad_kernel(Geom g, int V, int tiles, int batch, int per, int items, int flags,
+                                                      const float2* __restrict__ links, const float4* __restrict__ hin,
+                                                      const float4* __restrict__ delta, float* dW) {
+  constexpr int KP = kpad(CIN), MT = (2 * COUT + 15) / 16, MP = MT * 16, CH = CIN / 4;
+  extern __shared__ __align__(128) unsigned char smem[];
+  unsigned char* G = smem;                   // ROWS x KP
+  unsigned char* D = smem + ROWS * KP * 2;   // 2 x (ROWS x MP)
+  const int tid = threadIdx.x, d = tid >> 5, s = tid & 31;
+  if (d < 3) {  // the padding columns of both delta tiles
+    for (int c = 2 * COUT / 8; c < MP / 8; ++c)
+      for (int q = 0; q < 2; ++q)
+        *reinterpret_cast<uint4*>(D + q * (ROWS * MP * 2) + core_row<MP>(d * 32 + s, c)) = make_uint4(0, 0, 0, 0);
   }
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gid = lane >> 2, tig = lane & 3;
-  constexpr int MT = MP / 16, NT = KP / 8;
-  for (int t = warp; t < MT * NT; t += CT / 32) {
-    const int mt = t % MT, nt = t / MT;
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+  float acc[CH][MT][4];
 #pragma unroll
-    for (int ks = 0; ks < ROWS / 16; ++ks) {
-      const __nv_bfloat16* A0 = Dt + (size_t)(mt * 16 + gid) * DP + ks * 16 + 2 * tig;
-      const __nv_bfloat16* A1 = A0 + 8 * DP;
-      uint32_t a[4] = {ld_bf16x2(A0), ld_bf16x2(A1), ld_bf16x2(A0 + 8), ld_bf16x2(A1 + 8)};
-      // B (K = rows x N = k columns), col-major fragment: (k = 2 tig + {0,1}, n = gid)
-      const int col = nt * 8 + gid;
-      const int r0 = ks * 16 + 2 * tig;
-      uint32_t bb[2] = {pack_bf16(G[(size_t)r0 * GP + col], G[(size_t)(r0 + 1) * GP + col]),
-                        pack_bf16(G[(size_t)(r0 + 8) * GP + col], G[(size_t)(r0 + 9) * GP + col])};
-      mma_bf16(c, a, bb);
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int t = 0; t < MT; ++t)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[c][t][q] = 0.f;
+  const int parts = (batch + per - 1) / per;
+  int buf = 0;
+  for (int item = blockIdx.x; item < items; item += gridDim.x) {
+    int tile = item / parts, par = 1;
+    const int b0 = (item - tile * parts) * per, b1 = min(batch, b0 + per);
+    if (!(flags & OUT_ODD)) {
+      par = tile >= tiles ? 1 : 0;
+      tile -= par * tiles;
     }
+    const int i = tile * SITES + s;
+    const bool valid = i < g.Vh;
+    const int ic = valid ? i : g.Vh - 1;
+    const int j = par * g.Vh + ic;
+    const bool mine = !(flags & IN_ODD) || ((d == 0) == (par == 1));
+    const int n = neighbour(g, par, ic, d);
+    float2 m[9];
+    if (mine && d > 0) load_transport(m, links, V, j, n, d);
+    for (int b = b0; b < b1; ++b, buf ^= 1) {
+      unsigned char* Db = D + buf * (ROWS * MP * 2);
+      if (d < 3) {  // warp = colour: a row of delta, zero past the lattice's end
+        const float4* dl = delta + (size_t)b * V * planes(COUT) + j;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int n = mt * 16 + gid + 8 * half;
-      const int k = nt * 8 + 2 * tig;
-      if (n < 2 * COUT) {
-        atomicAdd(&dW[(size_t)n * KP + k], c[2 * half]);
-        atomicAdd(&dW[(size_t)n * KP + k + 1], c[2 * half + 1]);
+        for (int c = 0; c < COUT / 4; ++c) {
+          const float4 p = __ldg(dl + (size_t)(d * (COUT / 2) + 2 * c) * V);
+          const float4 q = __ldg(dl + (size_t)(d * (COUT / 2) + 2 * c + 1) * V);
+          uint4 w = make_uint4(bf16x2(p.x, p.y), bf16x2(p.z, p.w), bf16x2(q.x, q.y), bf16x2(q.z, q.w));
+          if (!valid) w = make_uint4(0, 0, 0, 0);
+          *reinterpret_cast<uint4*>(Db + core_row<MP>(d * 32 + s, c)) = w;
+        }
+      }
+      if (mine) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
+      __syncthreads();
+      if (mine) {
+        const uint32_t gs = smem_u32(G), ds = smem_u32(Db);
+#pragma unroll
+        for (int ks = 0; ks < ROWS / 16; ++ks) {
+          uint32_t a[MT][4];
+#pragma unroll
+          for (int t = 0; t < MT; ++t)
+            ldmatrix4_trans(a[t], ds + core_row<MP>(ks * 16 + (s >> 4) * 8 + (s & 7), t * 2 + ((s >> 3) & 1)));
+#pragma unroll
+          for (int c = 0; c < CH; ++c) {
+            uint32_t bb[2];
+            ldmatrix2_trans(bb, gs + core_row<KP>(ks * 16 + ((s >> 3) & 1) * 8 + (s & 7), d * CH + c));
+#pragma unroll
+            for (int t = 0; t < MT; ++t) mma_bf16(acc[c][t], a[t], bb);
+          }
+        }
+        __syncwarp();  // all lanes have read this warp's columns of G before the next gather
       }
     }
   }
+  const int gid = s >> 2, tig = s & 3;
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int t = 0; t < MT; ++t)
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int nn = t * 16 + gid + 8 * half, k = (d * CH + c) * 8 + 2 * tig;
+        if (nn < 2 * COUT) {
+          atomicAdd(&dW[(size_t)nn * KP + k], acc[c][t][2 * half]);
+          atomicAdd(&dW[(size_t)nn * KP + k + 1], acc[c][t][2 * half + 1]);
+        }
+      }
 }
 
-// odd-site spinor field (precision P) -> layer-0 activations (even sites zero)
-template <typename P>
-__global__ void embed_kernel(Geom g, int V, Spinor f, float2* act) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  const int b = blockIdx.y;
-  if (j >= V) return;
-  float2* out = act + ((size_t)b * V + j) * 12;
-  if (j < g.Vh) {
-    for (int k = 0; k < 12; ++k) out[k] = make_float2(0.f, 0.f);
-    return;
-  }
-  cplx<typename P::real> v[12];
-  load_spinor<P>(v, (const char*)f.v + (size_t)b * f.rhs_bytes, f.norm ? f.norm + (size_t)b * f.norm_rhs_stride : nullptr,
-                 j - g.Vh, f.stride);
-  for (int k = 0; k < 12; ++k) out[k] = make_float2((float)v[k].re, (float)v[k].im);
+// spinor components (spin * 3 + colour) of one site <-> the 6 planes of a 4-channel activation
+template <typename T>
+__device__ __forceinline__ void put_site(float4* act, int V, int j, const cplx<T> (&v)[12]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const cplx<T> x = v[(2 * q) * 3 + a], y = v[(2 * q + 1) * 3 + a];
+      act[(size_t)(a * 2 + q) * V + j] = make_float4((float)x.re, (float)y.re, (float)x.im, (float)y.im);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void get_site(const float4* act, int V, int j, cplx<T> (&v)[12]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const float4 w = act[(size_t)(a * 2 + q) * V + j];
+      v[(2 * q) * 3 + a] = {(T)w.x, (T)w.z};
+      v[(2 * q + 1) * 3 + a] = {(T)w.y, (T)w.w};
+    }
 }
 
+// odd-site spinor field (precision P) -> odd sites of the layer-0 activations
 template <typename P>
-__global__ void extract_kernel(Geom g, int V, const float2* act, Spinor f) {
+__global__ void embed_kernel(Geom g, int V, Spinor f, float4* act) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   if (i >= g.Vh) return;
-  const float2* src = act + ((size_t)b * V + g.Vh + i) * 12;
   cplx<typename P::real> v[12];
-  for (int k = 0; k < 12; ++k) v[k] = {(typename P::real)src[k].x, (typename P::real)src[k].y};
+  load_spinor<P>(v, (const char*)f.v + (size_t)b * f.rhs_bytes, f.norm ? f.norm + (size_t)b * f.norm_rhs_stride : nullptr,
+                 i, f.stride);
+  put_site(act + (size_t)b * V * planes(4), V, g.Vh + i, v);
+}
+
+template <typename P>
+__global__ void extract_kernel(Geom g, int V, const float4* act, Spinor f) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int b = blockIdx.y;
+  if (i >= g.Vh) return;
+  cplx<typename P::real> v[12];
+  get_site(act + (size_t)b * V * planes(4), V, g.Vh + i, v);
   store_spinor<P>((char*)f.v + (size_t)b * f.rhs_bytes, f.norm ? f.norm + (size_t)b * f.norm_rhs_stride : nullptr, i,
                   f.stride, v);
 }
 
-// canonical complex128 [V][12] (rhs b at offset b*V*12) -> activations, odd sites only
-__global__ void embed_canon_kernel(Geom g, int V, const double2* canon, float2* act) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// block sum of one double per thread (128 threads), valid in thread 0
+__device__ __forceinline__ double block_sum_128(double v) {
+  __shared__ double sh[4];
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return threadIdx.x == 0 ? (sh[0] + sh[1]) + (sh[2] + sh[3]) : 0.0;
+}
+
+// canonical complex128 [V][12] (rhs b at offset b*V*12) -> activations, odd sites only;
+// NORM: norm2[b] += |f_b|^2 over the odd sites, in FP64
+template <bool NORM>
+__global__ void __launch_bounds__(128) embed_canon_kernel(Geom g, int V, const double2* canon, float4* act,
+                                                          double* norm2) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
-  if (j >= V) return;
-  float2* out = act + ((size_t)b * V + j) * 12;
-  if (j < g.Vh) {
-    for (int k = 0; k < 12; ++k) out[k] = make_float2(0.f, 0.f);
-    return;
+  double sum = 0.0;
+  if (i < g.Vh) {
+    const Coord c = cb_coords(g, i, 1);
+    const double2* src = canon + ((size_t)b * V + full_index(g, c)) * 12;
+    cplx<double> v[12];
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      const double2 w = src[k];
+      v[k] = {w.x, w.y};
+      if (NORM) sum = fmadd(w.x, w.x, fmadd(w.y, w.y, sum));
+    }
+    put_site(act + (size_t)b * V * planes(4), V, g.Vh + i, v);
   }
-  const Coord c = eo_coords(g, j);
-  const double2* src = canon + ((size_t)b * V + full_index(g, c)) * 12;
-  for (int k = 0; k < 12; ++k) out[k] = make_float2((float)src[k].x, (float)src[k].y);
+  if constexpr (NORM) {
+    sum = block_sum_128(sum);
+    if (threadIdx.x == 0) atomicAdd(&norm2[b], sum);
+  }
 }
 
-__global__ void extract_canon_kernel(Geom g, int V, const float2* act, double2* canon) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// One thread per (canonical site, component): consecutive threads write consecutive 16-byte
+// components (one thread per site wrote 16 bytes of 32 different sectors per store instruction)
+__global__ void extract_canon_kernel(Geom g, int V, const float4* act, double2* canon) {
+  const long p = blockIdx.x * (long)blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
-  if (j >= V) return;
-  const Coord c = eo_coords(g, j);
-  double2* dst = canon + ((size_t)b * V + full_index(g, c)) * 12;
-  const float2* src = act + ((size_t)b * V + j) * 12;
-  for (int k = 0; k < 12; ++k)
-    dst[k] = j < g.Vh ? make_double2(0.0, 0.0) : make_double2((double)src[k].x, (double)src[k].y);
+  if (p >= (long)V * 12) return;
+  const int site = (int)(p / 12), k = (int)(p - (long)site * 12);
+  Coord c;
+  int r = site;
+  c.x[0] = r % g.L[0];
+  r /= g.L[0];
+  c.x[1] = r % g.L[1];
+  r /= g.L[1];
+  c.x[2] = r % g.L[2];
+  c.x[3] = r / g.L[2];
+  double2 v = make_double2(0.0, 0.0);
+  if ((c.x[0] + c.x[1] + c.x[2] + c.x[3]) & 1) {
+    const int spin = k / 3, a = k - spin * 3;
+    const float* w = reinterpret_cast<const float*>(
+        act + ((size_t)b * planes(4) + a * 2 + (spin >> 1)) * V + g.Vh + cb_index(g, c));
+    v = make_double2((double)w[spin & 1], (double)w[2 + (spin & 1)]);
+  }
+  canon[(size_t)b * V * 12 + p] = v;
 }
 
-// loss = sum_b sum_odd |y - e|^2 / |e|^2 ; delta = 2 (y - e) / |e|^2 on odd sites, 0 elsewhere
-__global__ void loss_kernel(Geom g, int V, const float2* y, const float2* e, const double* enorm2, float2* delta,
-                            double* partial) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// loss = sum_b sum_odd |y - e|^2 / |e|^2 ; delta = 2 (y - e) / |e|^2, all on the odd sites
+__global__ void __launch_bounds__(128) loss_kernel(Geom g, int V, const float4* y, const float4* e,
+                                                   const double* enorm2, float4* delta, double* partial) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int b = blockIdx.y;
   double l = 0.0;
-  if (j < V) {
-    const size_t o = ((size_t)b * V + j) * 12;
+  if (i < g.Vh) {
     const float inv = (float)(1.0 / enorm2[b]);
-    for (int k = 0; k < 12; ++k) {
-      float2 d = make_float2(0.f, 0.f);
-      if (j >= g.Vh) {
-        d = make_float2(y[o + k].x - e[o + k].x, y[o + k].y - e[o + k].y);
-        l += (double)(d.x * d.x + d.y * d.y) * inv;
-        d = make_float2(2.f * d.x * inv, 2.f * d.y * inv);
-      }
-      delta[o + k] = d;
+#pragma unroll
+    for (int q = 0; q < planes(4); ++q) {
+      const size_t o = ((size_t)b * planes(4) + q) * V + g.Vh + i;
+      const float4 p = y[o], t = e[o];
+      const float4 d = make_float4(p.x - t.x, p.y - t.y, p.z - t.z, p.w - t.w);
+      l += (double)(d.x * d.x + d.z * d.z) * inv;
+      l += (double)(d.y * d.y + d.w * d.w) * inv;
+      delta[o] = make_float4(2.f * d.x * inv, 2.f * d.y * inv, 2.f * d.z * inv, 2.f * d.w * inv);
     }
   }
-  __shared__ double sh[256];
-  sh[threadIdx.x] = l;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) atomicAdd(partial, sh[0]);
+  l = block_sum_128(l);
+  if (threadIdx.x == 0) atomicAdd(partial, l);
 }
 
+// canonical links -> FP32 planes [mu * 9 + entry][even-odd site]
 __global__ void links_kernel(Geom g, int V, const double2* canon, float2* links) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= V) return;
   const Coord c = eo_coords(g, j);
   const long s = full_index(g, c);
-  for (int m = 0; m < 4; ++m)
-    for (int k = 0; k < 9; ++k) {
-      const double2 v = canon[(s * 4 + m) * 9 + k];
-      links[((size_t)j * 4 + m) * 9 + k] = make_float2((float)v.x, (float)v.y);
-    }
+  for (int e = 0; e < 36; ++e) {
+    const double2 v = canon[s * 36 + e];
+    links[(size_t)e * V + j] = make_float2((float)v.x, (float)v.y);
+  }
+}
+
+// Work split of a layer over the grid: a block is a 32-site tile of one parity and up to `per`
+// right-hand sides, which share its transports and weights.  All of a batch in one block is best
+// while the tiles alone fill the chip; with fewer tiles than two waves (152 SMs x 3 blocks) the
+// batch is spread over more blocks.
+struct Split {
+  int tiles, blocks, per, parts;
+};
+Split split_of(const Geom& g, int batch, int flags) {
+  Split w;
+  w.tiles = (g.Vh + SITES - 1) / SITES;
+  w.blocks = (flags & OUT_ODD) ? w.tiles : 2 * w.tiles;
+  const int want = std::min(batch, std::max(1, 2 * 152 * 3 / w.blocks));
+  w.per = (batch + want - 1) / want;
+  w.parts = (batch + w.per - 1) / w.per;
+  return w;
 }
 
 template <int CIN, int COUT>
-void launch_layer(const Geom& g, int V, int batch, const float2* links, const float2* in, float2* out,
+void launch_layer(const Geom& g, int V, int batch, int flags, const float2* links, const float4* in, float4* out,
                   const __nv_bfloat16* W, cudaStream_t s) {
-  // tile G (128 rows) and weights W (nump rows), bf16 in the tensor cores' core-matrix layout
-  // (their bytes are a multiple of 128), then the staged transports (float2)
-  // G (96 rows) and W (npad rows) in the core-matrix layout, then the staged transports; at least
-  // the 128 rows x kpad that the MMA's A operand (and its B operand, ending earlier) spans
-  const size_t tile = (size_t)(ROWS * kpad(CIN) + npad(COUT) * kpad(CIN)) * 2;
-  const size_t span = (size_t)128 * kpad(CIN) * 2;
-  const size_t lkb = sizeof(float2) * SITES * 8 * 9;
-  const size_t smem = std::max(batch > 1 ? tile + lkb : tile, span);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(layer_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)std::max(tile + lkb, span));
-    attr = true;
-  }
-  dim3 grid((V + SITES - 1) / SITES);
-  layer_kernel<CIN, COUT><<<grid, CT, smem, s>>>(g, V, batch, links, in, out, W);
+  // G (96 rows) and W (npad rows) in the core-matrix layout, inside the 128 rows x kpad that the
+  // MMA's A operand (and its B operand, ending at the same row) spans
+  const size_t smem = (size_t)128 * kpad(CIN) * 2;
+  GBC_CUDA(cudaFuncSetAttribute(layer_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const Split w = split_of(g, batch, flags);
+  layer_kernel<CIN, COUT><<<dim3(w.blocks, w.parts), CT, smem, s>>>(g, V, w.tiles, batch, w.per, flags, links, in, out,
+                                                                    reinterpret_cast<const uint4*>(W));
   count_launch();
 }
 
 template <int CIN, int COUT>
-void launch_wgrad(const Geom& g, int V, int batch, const float2* links, const float2* in, const float2* delta,
-                  float* dW, cudaStream_t s) {
-  constexpr int MP = ((npad(COUT) + 15) / 16) * 16;
-  const size_t smem = (size_t)(ROWS * gpitch(CIN) + MP * DP) * 2;
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    attr = true;
-  }
-  dim3 grid((V + SITES - 1) / SITES, batch);
-  wgrad_kernel<CIN, COUT><<<grid, CT, smem, s>>>(g, V, links, in, delta, dW);
+void launch_wgrad(const Geom& g, int V, int batch, int flags, const float2* links, const float4* in,
+                  const float4* delta, float* dW, cudaStream_t s) {
+  constexpr int MP = ((2 * COUT + 15) / 16) * 16;
+  const size_t smem = (size_t)ROWS * (kpad(CIN) + 2 * MP) * 2;
+  GBC_CUDA(cudaFuncSetAttribute(wgrad_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const Split w = split_of(g, batch, flags);
+  const int items = w.blocks * w.parts;
+  // two resident blocks per SM walk the items (their sums live in registers)
+  wgrad_kernel<CIN, COUT><<<std::min(items, 2 * 152), CT, smem, s>>>(g, V, w.tiles, batch, w.per, items, flags, links,
+                                                                     in, delta, dW);
   count_launch();
 }
 
-void layer(const Geom& g, int V, int batch, int cin, int cout, const float2* links, const float2* in, float2* out,
-           const __nv_bfloat16* W, cudaStream_t s) {
-  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, links, in, out, W, s);
-  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, links, in, out, W, s);
-  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, links, in, out, W, s);
-  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, links, in, out, W, s);
+void layer(const Geom& g, int V, int batch, int cin, int cout, int flags, const float2* links, const float4* in,
+           float4* out, const __nv_bfloat16* W, cudaStream_t s) {
+  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, flags, links, in, out, W, s);
+  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, flags, links, in, out, W, s);
+  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, flags, links, in, out, W, s);
+  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, flags, links, in, out, W, s);
   else throw std::string("network layer shape not compiled");
 }
 
-void wgrad(const Geom& g, int V, int batch, int cin, int cout, const float2* links, const float2* in,
-           const float2* delta, float* dW, cudaStream_t s) {
-  if (cin == 4 && cout == 12) launch_wgrad<4, 12>(g, V, batch, links, in, delta, dW, s);
-  else if (cin == 12 && cout == 12) launch_wgrad<12, 12>(g, V, batch, links, in, delta, dW, s);
-  else if (cin == 12 && cout == 4) launch_wgrad<12, 4>(g, V, batch, links, in, delta, dW, s);
-  else if (cin == 4 && cout == 4) launch_wgrad<4, 4>(g, V, batch, links, in, delta, dW, s);
+void wgrad(const Geom& g, int V, int batch, int cin, int cout, int flags, const float2* links, const float4* in,
+           const float4* delta, float* dW, cudaStream_t s) {
+  if (cin == 4 && cout == 12) launch_wgrad<4, 12>(g, V, batch, flags, links, in, delta, dW, s);
+  else if (cin == 12 && cout == 12) launch_wgrad<12, 12>(g, V, batch, flags, links, in, delta, dW, s);
+  else if (cin == 12 && cout == 4) launch_wgrad<12, 4>(g, V, batch, flags, links, in, delta, dW, s);
+  else if (cin == 4 && cout == 4) launch_wgrad<4, 4>(g, V, batch, flags, links, in, delta, dW, s);
   else throw std::string("network layer shape not compiled");
 }
 
@@ -632,8 +693,9 @@ void Cnn::init(int hidden_, int layers_, unsigned long long seed) {
   dirty = true;
 }
 
+// Real form of a layer's weights in the MMA's order (comp) and core-matrix layout: rows n = comp(o, .)
+// of the outputs, columns k = (d * C_in + i) * 2 + re/im.
 static void real_form(const std::vector<cf>& Wc, int ci, int co, bool adjoint, std::vector<__nv_bfloat16>& out) {
-  // forward: rows 2*COUT (re/im of output o), K = (d*CIN + i)*2 + re/im
   // adjoint: out channels = ci, in channels = co, W'_d = (W_{swap d})^H
   const int oc = adjoint ? ci : co, ic = adjoint ? co : ci;
   const int KP = kpad(ic), NP = npad(oc);
@@ -643,11 +705,14 @@ static void real_form(const std::vector<cf>& Wc, int ci, int co, bool adjoint, s
     for (int o = 0; o < oc; ++o)
       for (int i = 0; i < ic; ++i) {
         cf w = adjoint ? std::conj(Wc[((size_t)ds * co + i) * ci + o]) : Wc[((size_t)d * co + o) * ci + i];
-        const int k = (d * ic + i) * 2;
-        out[(size_t)(2 * o) * KP + k] = __float2bfloat16(w.real());
-        out[(size_t)(2 * o) * KP + k + 1] = __float2bfloat16(-w.imag());
-        out[(size_t)(2 * o + 1) * KP + k] = __float2bfloat16(w.imag());
-        out[(size_t)(2 * o + 1) * KP + k + 1] = __float2bfloat16(w.real());
+        auto at = [&](int no, int ki) -> __nv_bfloat16& {
+          const int n = comp(o, no), k = (d * ic + i) * 2 + ki;
+          return out[(size_t)(n >> 3) * (KP * 8) + (k >> 3) * 64 + (n & 7) * 8 + (k & 7)];
+        };
+        at(0, 0) = __float2bfloat16(w.real());
+        at(0, 1) = __float2bfloat16(-w.imag());
+        at(1, 0) = __float2bfloat16(w.imag());
+        at(1, 1) = __float2bfloat16(w.real());
       }
   }
 }
@@ -661,7 +726,6 @@ void Cnn::upload(cudaStream_t s) {
     if (!dW[l]) {
       GBC_CUDA(cudaMalloc(&dW[l], a.size() * 2));
       GBC_CUDA(cudaMalloc(&dWadj[l], b.size() * 2));
-      GBC_CUDA(cudaMalloc(&dG[l], sizeof(float) * (size_t)npad(cout(l)) * kpad(cin(l))));
     }
     GBC_CUDA(cudaMemcpyAsync(dW[l], a.data(), a.size() * 2, cudaMemcpyHostToDevice, s));
     GBC_CUDA(cudaMemcpyAsync(dWadj[l], b.data(), b.size() * 2, cudaMemcpyHostToDevice, s));
@@ -674,18 +738,17 @@ void Cnn::release() {
   for (int l = 0; l < 8; ++l) {
     if (dW[l]) cudaFree(dW[l]);
     if (dWadj[l]) cudaFree(dWadj[l]);
-    if (dG[l]) cudaFree(dG[l]);
     dW[l] = dWadj[l] = nullptr;
-    dG[l] = nullptr;
   }
   for (auto& p : act) if (p) cudaFree(p);
   act.clear();
-  if (links) cudaFree(links);
+  for (void* p : {(void*)links, (void*)delta[0], (void*)delta[1], (void*)target, (void*)dG, (void*)norms})
+    if (p) cudaFree(p);
   links = nullptr;
-  if (delta[0]) cudaFree(delta[0]);
-  if (delta[1]) cudaFree(delta[1]);
-  delta[0] = delta[1] = nullptr;
-  act_batch = 0;
+  delta[0] = delta[1] = target = nullptr;
+  dG = nullptr;
+  norms = nullptr;
+  act_batch = train_batch = 0;
 }
 
 void Cnn::ensure(gbc_ctx* c, int batch) {
@@ -697,24 +760,49 @@ void Cnn::ensure(gbc_ctx* c, int batch) {
     links_version = c->gauge_version;
   }
   if (act_batch < batch) {
+    act_batch = 0;
     for (auto& p : act) if (p) cudaFree(p);
     act.assign(nlayers + 1, nullptr);
-    for (int l = 0; l <= nlayers; ++l) {
-      const int ch = l == 0 ? 4 : cout(l - 1);
-      GBC_CUDA(cudaMalloc(&act[l], sizeof(float2) * (size_t)batch * V * std::max(ch, 12) * 3));
-    }
-    for (int q = 0; q < 2; ++q) {
-      if (delta[q]) cudaFree(delta[q]);
-      GBC_CUDA(cudaMalloc(&delta[q], sizeof(float2) * (size_t)batch * V * std::max(hidden, 4) * 3));
-    }
+    for (int l = 0; l <= nlayers; ++l)
+      GBC_CUDA(cudaMalloc(&act[l], sizeof(float4) * (size_t)batch * V * planes(l == 0 ? 4 : cout(l - 1))));
     act_batch = batch;
   }
   upload(c->stream);
 }
 
+// Workspaces of the training step: targets, back-propagated deltas, the weight gradients of all
+// layers in one buffer, and the target norms with the loss behind them.
+void Cnn::ensure_train(gbc_ctx* c, int batch) {
+  ensure(c, batch);
+  if (!dG) GBC_CUDA(cudaMalloc(&dG, sizeof(float) * grad_offset(nlayers)));
+  if (train_batch >= batch) return;
+  train_batch = 0;
+  for (float4** p : {&delta[0], &delta[1], &target}) {
+    if (*p) cudaFree(*p);
+    *p = nullptr;
+  }
+  if (norms) cudaFree(norms);
+  norms = nullptr;
+  const size_t V = (size_t)c->V;
+  for (int q = 0; q < 2; ++q) GBC_CUDA(cudaMalloc(&delta[q], sizeof(float4) * batch * V * planes(hidden)));
+  GBC_CUDA(cudaMalloc(&target, sizeof(float4) * batch * V * planes(4)));
+  GBC_CUDA(cudaMalloc(&norms, sizeof(double) * (batch + 1)));
+  train_batch = batch;
+}
+
+size_t Cnn::grad_offset(int l) const {
+  size_t n = 0;
+  for (int k = 0; k < l; ++k) n += (size_t)npad(cout(k)) * kpad(cin(k));
+  return n;
+}
+
+// The network's input is zero on the even sites and only its odd output sites are wanted: the
+// first layer skips the zero terms, the last the even sites.
 void Cnn::forward(gbc_ctx* c, int batch) {
   const int V = (int)c->V;
-  for (int l = 0; l < nlayers; ++l) layer(c->g, V, batch, cin(l), cout(l), links, act[l], act[l + 1], dW[l], c->stream);
+  for (int l = 0; l < nlayers; ++l)
+    layer(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (l == nlayers - 1 ? OUT_ODD : 0), links, act[l],
+          act[l + 1], dW[l], c->stream);
 }
 
 // A layer whose wait for its tensor-core results gave up (it then frees its tensor memory and
@@ -730,30 +818,28 @@ static void check_tc_waits(cudaStream_t s) {
   }
 }
 
-double Cnn::loss_and_grad(gbc_ctx* c, int batch, const float2* target, const double* enorm2) {
+double Cnn::loss_and_grad(gbc_ctx* c, int batch) {
   const int V = (int)c->V;
   cudaStream_t s = c->stream;
   forward(c, batch);
-  double* dl = nullptr;
-  GBC_CUDA(cudaMalloc(&dl, sizeof(double)));
+  double* dl = norms + batch;
   GBC_CUDA(cudaMemsetAsync(dl, 0, sizeof(double), s));
-  dim3 grid((V + 255) / 256, batch);
-  loss_kernel<<<grid, 256, 0, s>>>(c->g, V, act[nlayers], target, enorm2, delta[0], dl);
+  loss_kernel<<<dim3((c->g.Vh + 127) / 128, batch), 128, 0, s>>>(c->g, V, act[nlayers], target, norms, delta[0], dl);
   count_launch();
-  for (int l = 0; l < nlayers; ++l)
-    GBC_CUDA(cudaMemsetAsync(dG[l], 0, sizeof(float) * (size_t)npad(cout(l)) * kpad(cin(l)), s));
+  GBC_CUDA(cudaMemsetAsync(dG, 0, sizeof(float) * grad_offset(nlayers), s));
   int cur = 0;
   for (int l = nlayers - 1; l >= 0; --l) {
-    wgrad(c->g, V, batch, cin(l), cout(l), links, act[l], delta[cur], dG[l], s);
+    // delta of the last layer lives on the odd sites, the first layer's input too
+    const bool last = l == nlayers - 1;
+    wgrad(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (last ? OUT_ODD : 0), links, act[l], delta[cur],
+          dG + grad_offset(l), s);
     if (l > 0) {
-      layer(c->g, V, batch, cout(l), cin(l), links, delta[cur], delta[1 - cur], dWadj[l], s);
+      layer(c->g, V, batch, cout(l), cin(l), last ? IN_ODD : 0, links, delta[cur], delta[1 - cur], dWadj[l], s);
       cur = 1 - cur;
     }
   }
   double loss = 0;
   GBC_CUDA(cudaMemcpyAsync(&loss, dl, sizeof(double), cudaMemcpyDeviceToHost, s));
-  GBC_CUDA(cudaStreamSynchronize(s));
-  cudaFree(dl);
   check_tc_waits(s);
   return loss;
 }
@@ -761,19 +847,18 @@ double Cnn::loss_and_grad(gbc_ctx* c, int batch, const float2* target, const dou
 // complex gradient dL/dRe W + i dL/dIm W from the real-form gradient
 void Cnn::download_grad(cudaStream_t s, std::vector<std::vector<cf>>& grad) {
   grad.assign(nlayers, {});
+  std::vector<float> all(grad_offset(nlayers));
+  GBC_CUDA(cudaMemcpyAsync(all.data(), dG, all.size() * 4, cudaMemcpyDeviceToHost, s));
+  GBC_CUDA(cudaStreamSynchronize(s));
   for (int l = 0; l < nlayers; ++l) {
     const int ci = cin(l), co = cout(l), KP = kpad(ci);
-    std::vector<float> gr((size_t)npad(co) * KP);
-    GBC_CUDA(cudaMemcpyAsync(gr.data(), dG[l], gr.size() * 4, cudaMemcpyDeviceToHost, s));
-    GBC_CUDA(cudaStreamSynchronize(s));
+    const float* gr = all.data() + grad_offset(l);
     grad[l].assign((size_t)9 * co * ci, cf(0, 0));
     for (int d = 0; d < 9; ++d)
       for (int o = 0; o < co; ++o)
         for (int i = 0; i < ci; ++i) {
-          const int k = (d * ci + i) * 2;
-          const float dre = gr[(size_t)(2 * o) * KP + k] + gr[(size_t)(2 * o + 1) * KP + k + 1];
-          const float dim = gr[(size_t)(2 * o + 1) * KP + k] - gr[(size_t)(2 * o) * KP + k + 1];
-          grad[l][((size_t)d * co + o) * ci + i] = cf(dre, dim);
+          auto at = [&](int no, int ki) { return gr[(size_t)comp(o, no) * KP + (d * ci + i) * 2 + ki]; };
+          grad[l][((size_t)d * co + o) * ci + i] = cf(at(0, 0) + at(1, 1), at(1, 0) - at(0, 1));
         }
   }
 }
@@ -870,31 +955,36 @@ int Cnn::load(const std::string& path) {
 void cnn_apply_spinor(gbc_ctx* c, Cnn& net, const Spinor& in, const Spinor& out) {
   const int V = (int)c->V;
   net.ensure(c, in.nrhs);
-  dim3 grid((V + 127) / 128, in.nrhs);
+  const dim3 grid((c->g.Vh + 127) / 128, in.nrhs);
   if (in.prec == PREC_DOUBLE) embed_kernel<PrecD><<<grid, 128, 0, c->stream>>>(c->g, V, in, net.act[0]);
   else if (in.prec == PREC_SINGLE) embed_kernel<PrecS><<<grid, 128, 0, c->stream>>>(c->g, V, in, net.act[0]);
   else embed_kernel<PrecH><<<grid, 128, 0, c->stream>>>(c->g, V, in, net.act[0]);
   count_launch();
   net.forward(c, in.nrhs);
-  dim3 g2((c->g.Vh + 127) / 128, in.nrhs);
-  if (out.prec == PREC_DOUBLE) extract_kernel<PrecD><<<g2, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
-  else if (out.prec == PREC_SINGLE) extract_kernel<PrecS><<<g2, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
-  else extract_kernel<PrecH><<<g2, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
+  if (out.prec == PREC_DOUBLE) extract_kernel<PrecD><<<grid, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
+  else if (out.prec == PREC_SINGLE) extract_kernel<PrecS><<<grid, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
+  else extract_kernel<PrecH><<<grid, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
   count_launch();
   check_tc_waits(c->stream);
 }
 
-void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float2* act) {
+void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float4* act, double* norm2) {
   const int V = (int)c->V;
-  dim3 grid((V + 127) / 128, batch);
-  embed_canon_kernel<<<grid, 128, 0, c->stream>>>(c->g, V, reinterpret_cast<const double2*>(canon_dev), act);
+  const dim3 grid((c->g.Vh + 127) / 128, batch);
+  const double2* src = reinterpret_cast<const double2*>(canon_dev);
+  if (norm2) {
+    GBC_CUDA(cudaMemsetAsync(norm2, 0, sizeof(double) * batch, c->stream));
+    embed_canon_kernel<true><<<grid, 128, 0, c->stream>>>(c->g, V, src, act, norm2);
+  } else {
+    embed_canon_kernel<false><<<grid, 128, 0, c->stream>>>(c->g, V, src, act, nullptr);
+  }
   count_launch();
 }
 
-void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float2* act, double* canon_dev) {
+void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float4* act, double* canon_dev) {
   const int V = (int)c->V;
-  dim3 grid((V + 127) / 128, batch);
-  extract_canon_kernel<<<grid, 128, 0, c->stream>>>(c->g, V, act, reinterpret_cast<double2*>(canon_dev));
+  const dim3 grid((unsigned)(((long)V * 12 + 255) / 256), batch);
+  extract_canon_kernel<<<grid, 256, 0, c->stream>>>(c->g, V, act, reinterpret_cast<double2*>(canon_dev));
   count_launch();
 }
 

@@ -23,13 +23,15 @@ struct Cnn {
   long step = 0;
   bool dirty = true;
 
-  __nv_bfloat16* dW[8] = {nullptr};     // real form [npad(cout)][kpad(cin)]
+  __nv_bfloat16* dW[8] = {nullptr};     // real form, npad(cout) x kpad(cin) in core-matrix layout
   __nv_bfloat16* dWadj[8] = {nullptr};  // input-gradient form
-  float* dG[8] = {nullptr};             // real-form weight gradients
-  std::vector<float2*> act;             // activations per layer boundary, [batch][V][ch][3]
-  float2* delta[2] = {nullptr, nullptr};
-  int act_batch = 0;
-  float2* links = nullptr;              // FP32 links, even-odd order [V][4][9]
+  float* dG = nullptr;                  // real-form weight gradients, layer l at grad_offset(l)
+  std::vector<float4*> act;             // activations per layer boundary, [batch][plane][V]
+  float4* delta[2] = {nullptr, nullptr};
+  float4* target = nullptr;             // training targets, as 4-channel activations
+  double* norms = nullptr;              // |target_b|^2, then the loss
+  int act_batch = 0, train_batch = 0;
+  float2* links = nullptr;              // FP32 links, planes [4 * 9][V] in even-odd order
   long links_version = -1;
 
   int cin(int l) const;
@@ -37,9 +39,12 @@ struct Cnn {
   void init(int hidden, int layers, unsigned long long seed);
   void upload(cudaStream_t s);
   void ensure(gbc_ctx* c, int batch);
+  void ensure_train(gbc_ctx* c, int batch);
+  size_t grad_offset(int l) const;
   void forward(gbc_ctx* c, int batch);
-  // forward + backward of sum_b |y_b - e_b|^2 / |e_b|^2 (odd sites); gradients left in dG
-  double loss_and_grad(gbc_ctx* c, int batch, const float2* target, const double* enorm2);
+  // forward + backward of sum_b |y_b - e_b|^2 / |e_b|^2 (odd sites; e in target, |e|^2 in norms);
+  // gradients left in dG
+  double loss_and_grad(gbc_ctx* c, int batch);
   void download_grad(cudaStream_t s, std::vector<std::vector<std::complex<float>>>& grad);
   void adam(const std::vector<std::vector<std::complex<float>>>& grad, double lr);
   bool save(const std::string& path) const;
@@ -48,7 +53,8 @@ struct Cnn {
 };
 
 void cnn_apply_spinor(gbc_ctx* c, Cnn& net, const Spinor& in, const Spinor& out);
-void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float2* act);
-void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float2* act, double* canon_dev);
+// norm2 (may be null): |f_b|^2 of each field over the odd sites, summed in FP64
+void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float4* act, double* norm2 = nullptr);
+void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float4* act, double* canon_dev);
 
 }  // namespace gbc

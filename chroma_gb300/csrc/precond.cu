@@ -52,29 +52,6 @@ int guard(gbc_ctx* c, F&& f) {
   }
 }
 
-// |e|^2 over the odd sites of nb canonical host fields
-std::vector<double> odd_norms(const gbc_ctx* c, const double* f, int nb) {
-  std::vector<double> n(nb, 0.0);
-  const long V = c->V;
-  for (int b = 0; b < nb; ++b) {
-    const double* p = f + (size_t)b * V * 24;
-    double s = 0;
-    for (long site = 0; site < V; ++site) {
-      long r = site;
-      int x = r % c->dims[0];
-      r /= c->dims[0];
-      int y = r % c->dims[1];
-      r /= c->dims[1];
-      int z = r % c->dims[2];
-      int t = (int)(r / c->dims[2]);
-      if (((x + y + z + t) & 1) == 0) continue;
-      for (int k = 0; k < 24; ++k) s += p[site * 24 + k] * p[site * 24 + k];
-    }
-    n[b] = s;
-  }
-  return n;
-}
-
 }  // namespace
 
 extern "C" {
@@ -172,20 +149,12 @@ int gbc_precond_loss_grad(gbc_ctx* c, int nb, const double* in, const double* ta
     Cnn& n = *net_of(c);
     ensure_stage(c, nb);
     const size_t bytes = (size_t)nb * c->V * 24 * sizeof(double);
-    n.ensure(c, nb);
-    std::vector<double> en = odd_norms(c, target, nb);
-    double* d_en = nullptr;
-    float2* tgt = nullptr;
-    GBC_CUDA(cudaMalloc(&d_en, sizeof(double) * nb));
-    GBC_CUDA(cudaMalloc(&tgt, sizeof(float2) * (size_t)nb * c->V * 12));
-    GBC_CUDA(cudaMemcpyAsync(d_en, en.data(), sizeof(double) * nb, cudaMemcpyHostToDevice, c->stream));
+    n.ensure_train(c, nb);
     GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], in, bytes, cudaMemcpyHostToDevice, c->stream));
     GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], target, bytes, cudaMemcpyHostToDevice, c->stream));
     cnn_embed_canon(c, n, nb, c->d_stage[0], n.act[0]);
-    cnn_embed_canon(c, n, nb, c->d_stage[1], tgt);
-    *loss = n.loss_and_grad(c, nb, tgt, d_en);
-    cudaFree(d_en);
-    cudaFree(tgt);
+    cnn_embed_canon(c, n, nb, c->d_stage[1], n.target, n.norms);
+    *loss = n.loss_and_grad(c, nb);
     if (grad) {
       std::vector<std::vector<std::complex<float>>> g;
       n.download_grad(c->stream, g);
@@ -213,16 +182,11 @@ int gbc_precond_train(gbc_ctx* c, int nsamples, const double* in, const double* 
     batch = std::min(batch, nsamples);
     const size_t per = (size_t)c->V * 24;
     ensure_stage(c, batch);
-    n.ensure(c, batch);
-    std::vector<double> en = odd_norms(c, target, nsamples);
-    double* d_en = nullptr;
-    float2* tgt = nullptr;
-    GBC_CUDA(cudaMalloc(&d_en, sizeof(double) * batch));
-    GBC_CUDA(cudaMalloc(&tgt, sizeof(float2) * (size_t)batch * c->V * 12));
+    n.ensure_train(c, batch);
     std::vector<int> order(nsamples);
     std::iota(order.begin(), order.end(), 0);
     std::mt19937_64 rng(seed);
-    std::vector<double> hin(per * batch), htg(per * batch), hen(batch);
+    std::vector<double> hin(per * batch), htg(per * batch);
     for (int ep = 0; ep < epochs; ++ep) {
       std::shuffle(order.begin(), order.end(), rng);
       double tot = 0;
@@ -231,17 +195,15 @@ int gbc_precond_train(gbc_ctx* c, int nsamples, const double* in, const double* 
           const int q = order[s0 + b];
           std::memcpy(&hin[per * b], in + per * q, per * sizeof(double));
           std::memcpy(&htg[per * b], target + per * q, per * sizeof(double));
-          hen[b] = en[q];
         }
         GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], hin.data(), per * batch * sizeof(double), cudaMemcpyHostToDevice,
                                  c->stream));
         GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], htg.data(), per * batch * sizeof(double), cudaMemcpyHostToDevice,
                                  c->stream));
-        GBC_CUDA(cudaMemcpyAsync(d_en, hen.data(), sizeof(double) * batch, cudaMemcpyHostToDevice, c->stream));
         n.upload(c->stream);
         cnn_embed_canon(c, n, batch, c->d_stage[0], n.act[0]);
-        cnn_embed_canon(c, n, batch, c->d_stage[1], tgt);
-        tot += n.loss_and_grad(c, batch, tgt, d_en);
+        cnn_embed_canon(c, n, batch, c->d_stage[1], n.target, n.norms);
+        tot += n.loss_and_grad(c, batch);
         std::vector<std::vector<std::complex<float>>> g;
         n.download_grad(c->stream, g);
         for (auto& w : g)
@@ -251,8 +213,6 @@ int gbc_precond_train(gbc_ctx* c, int nsamples, const double* in, const double* 
       if (loss_per_epoch) loss_per_epoch[ep] = tot / (nsamples / batch * batch);
     }
     n.upload(c->stream);
-    cudaFree(d_en);
-    cudaFree(tgt);
     return GBC_OK;
   });
 }
