@@ -435,9 +435,14 @@ void hop(gbc_ctx* c, int prec, int out_parity, int mode, bool dag, double a, con
     h.aux = c->hop_aux.v;
     h.aux_rhs_bytes = c->hop_aux.rhs_bytes;
   }
-  const HopShape sh = kHopShapes[tuned_shape(c, prec, f.recon, mode, dag, reduce, h)];
-  if (hop_blocks(sh, h.g.Vh) > c->part_stride) throw std::string("partials buffer too small");
-  int nb = hop_launch(prec, f.recon, mode, dag, reduce, h, sh, c->stream);
+  int nb;
+  if (prec == PREC_DOUBLE && hop_split(h.g.Vh, h.nrhs)) {
+    nb = hop_split_launch(mode, dag, reduce, h, hop_split_sites(h.g.Vh, h.nrhs), c->stream);
+  } else {
+    const HopShape sh = kHopShapes[tuned_shape(c, prec, f.recon, mode, dag, reduce, h)];
+    if (hop_blocks(sh, h.g.Vh) > c->part_stride) throw std::string("partials buffer too small");
+    nb = hop_launch(prec, f.recon, mode, dag, reduce, h, sh, c->stream);
+  }
   if (nb < 0) throw std::string("hopping kernel variant not compiled");
   count_launch();
   GBC_CUDA(cudaGetLastError());
@@ -595,6 +600,8 @@ int gbc_create(gbc_ctx** out, const gbc_geom* geom, const gbc_action* act, const
     if (noalloc_reserve() != GBC_OK) throw CudaError{cudaErrorMemoryAllocation, "noalloc scratch reservation"};
     // reduction partials: the largest grid is the hopping kernel with 16 sites per block
     c->part_stride = (g.Vh + 15) / 16;
+    // (the split FP64 kernel goes down to 8 sites per block while those are few)
+    if (hop_split_sites(g.Vh, 1) == 8) c->part_stride = (g.Vh + 7) / 8;
     if (c->part_stride < blas_blocks(g)) c->part_stride = blas_blocks(g);
     GBC_CUDA(cudaMalloc(&c->d_partials, sizeof(double) * 3 * c->max_rhs * (size_t)c->part_stride));
     GBC_CUDA(cudaMalloc(&c->d_result, sizeof(double) * 3 * c->max_rhs));

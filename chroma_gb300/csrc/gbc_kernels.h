@@ -109,6 +109,22 @@ int hop_launch_d(int recon, int mode, bool dag, int reduce, const HopArgs& a, Ho
 int hop_launch_s(int recon, int mode, bool dag, int reduce, const HopArgs& a, HopShape sh, cudaStream_t s);
 int hop_launch_h(int recon, int mode, bool dag, int reduce, const HopArgs& a, HopShape sh, cudaStream_t s);
 
+// FP64 with the hops of a site split over 8 threads, blocks of `sites` (8, 16 or 32) sites of one
+// right-hand side; reduce as in hop_launch.  Returns the blocks per right-hand side.
+int hop_split_launch(int mode, bool dag, int reduce, const HopArgs& a, int sites, cudaStream_t s);
+// Where the split kernel runs.  Both are bound by the FP64 pipe; the split one spreads small lattices
+// over all SMs, the other shares links between the right-hand sides of a block.  FP64 M~ on a GB300, split
+// against hop_kernel: 8^4 33 / 93 us, 16^3 x 32 291 / 324 us (4 right-hand sides 1065 / 1088 us), 24^3 x 48
+// 1358 / 1391 us; 16^3 x 32 with 8 right-hand sides 2112 / 2083 us, 32^3 x 64 with 12 50.2 / 49.5 ms.
+inline bool hop_split(int Vh, int nrhs) { return (long)Vh * nrhs <= 400000; }
+// Sites per block of the split FP64 kernel: the largest block that still gives every SM four of
+// them, so that the tail of the grid stays short.
+inline int hop_split_sites(int Vh, int nrhs) {
+  for (int sites : {32, 16})
+    if ((long)((Vh + sites - 1) / sites) * nrhs >= 4 * 152) return sites;
+  return 8;
+}
+
 // One launch over several lattices: args[l] in device memory, work[b] = (lattice, 128-site block).
 int hop_multi_launch_d(int recon, int mode, bool dag, int reduce, const HopArgs* args, const int2* work, int nwork,
                        cudaStream_t s);

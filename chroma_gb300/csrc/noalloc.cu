@@ -16,6 +16,7 @@
 
 #include "../../include/gbclover.h"
 #include "dslash.cuh"
+#include "dslash_split.cuh"
 
 namespace gbc {
 namespace {
@@ -27,148 +28,67 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 double2* g_scratch_ptr[kMaxDevices] = {nullptr};
 
-struct CanonGeom {
-  int L[4];
-  int Lxh;
-  int Vh;
+// Field access of split_site (dslash_split.cuh) in the canonical layouts; the even intermediate is
+// the scratch array, indexed by checkerboard site.
+template <int PARITY>
+struct CanonField {
+  Geom g;
+  const double2* links;
+  const double* clov;
+  const double2* psi;
+  double2* scratch;
+  double2* dst;
+  __device__ __forceinline__ const Geom& geom() const { return g; }
+  __device__ __forceinline__ int parity() const { return PARITY; }
+  __device__ __forceinline__ double2 in(const Coord& n, int ni, int k) const {
+    return PARITY == 0 ? psi[(size_t)full_index(g, n) * 12 + k] : scratch[(size_t)ni * 12 + k];
+  }
+  __device__ __forceinline__ double2 link(const Coord& c, int, const Coord& n, int, int mu, bool fwd, int e) const {
+    return links[((size_t)full_index(g, fwd ? c : n) * 4 + mu) * 9 + e];
+  }
+  __device__ __forceinline__ double diag(const Coord& c, int, int b, int i) const {
+    return clov[(size_t)full_index(g, c) * 72 + 6 * b + i];
+  }
+  __device__ __forceinline__ double2 offd(const Coord& c, int, int b, int k) const {
+    const double* p = clov + (size_t)full_index(g, c) * 72 + 12 + 30 * b + 2 * k;  // 8-byte aligned
+    return make_double2(p[0], p[1]);
+  }
+  __device__ __forceinline__ double2 self(const Coord& c, int, int k) const {
+    return psi[(size_t)full_index(g, c) * 12 + k];
+  }
+  __device__ __forceinline__ double2 aux(int, int) const { return make_double2(0.0, 0.0); }
+  __device__ __forceinline__ void out(const Coord& c, int idx, int k, int im, double v) const {
+    double2* p = PARITY == 0 ? scratch + (size_t)idx * 12 : dst + (size_t)full_index(g, c) * 12;
+    reinterpret_cast<double*>(p + k)[im] = v;
+  }
 };
 
-__device__ __forceinline__ Coord cg_coords(const CanonGeom& g, int i, int parity) {
-  Coord c;
-  int xh = i % g.Lxh;
-  int r = i / g.Lxh;
-  c.x[1] = r % g.L[1];
-  r /= g.L[1];
-  c.x[2] = r % g.L[2];
-  c.x[3] = r / g.L[2];
-  c.x[0] = 2 * xh + ((parity + c.x[1] + c.x[2] + c.x[3]) & 1);
-  return c;
-}
-__device__ __forceinline__ long cg_full(const CanonGeom& g, const Coord& c) {
-  return c.x[0] + (long)g.L[0] * (c.x[1] + (long)g.L[1] * (c.x[2] + (long)g.L[2] * c.x[3]));
-}
-__device__ __forceinline__ int cg_half(const CanonGeom& g, const Coord& c) {
-  return (c.x[0] >> 1) + g.Lxh * (c.x[1] + g.L[1] * (c.x[2] + g.L[2] * c.x[3]));
-}
-
-__device__ __forceinline__ void ld_site(cplx<double> (&v)[12], const double2* p) {
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    double2 w = p[k];
-    v[k] = {w.x, w.y};
-  }
-}
-__device__ __forceinline__ void ld_link(cplx<double> (&u)[9], const double2* p) {
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    double2 w = p[k];
-    u[k] = {w.x, w.y};
-  }
-}
-// y = T x for the two chiral blocks of one canonical packed site {diag[2][6], offd[2][15]}
-__device__ __forceinline__ void clover_site(cplx<double> (&y)[12], const double* t, const cplx<double> (&x)[12]) {
-#pragma unroll
-  for (int b = 0; b < 2; ++b) {
-    double d[6];
-    cplx<double> o[15], xb[6], yb[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) d[k] = t[6 * b + k];
-#pragma unroll
-    for (int k = 0; k < 15; ++k) o[k] = {t[12 + 30 * b + 2 * k], t[13 + 30 * b + 2 * k]};
-#pragma unroll
-    for (int k = 0; k < 6; ++k) xb[k] = x[6 * b + k];
-    clover_block_mul(yb, d, o, xb);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) y[6 * b + k] = yb[k];
-  }
-}
-
-// D' psi at site c (parity of c), reading psi from the canonical array (other parity) or, for
-// the second half, from the even scratch indexed by checkerboard index.
-template <bool DAG, bool FROM_SCRATCH>
-__device__ void hop_canon(cplx<double> (&acc)[12], const CanonGeom& g, const Coord& c, const double2* links,
-                          const double2* psi, const double2* scratch) {
-#pragma unroll
-  for (int k = 0; k < 12; ++k) acc[k] = {0.0, 0.0};
-  cplx<double> s[12], h[2][3], uh[2][3], u[9];
-  const long self = cg_full(g, c);
-#pragma unroll
-  for (int mu = 0; mu < 4; ++mu) {
-    Coord n = c;
-    n.x[mu] = c.x[mu] + 1 == g.L[mu] ? 0 : c.x[mu] + 1;
-    if (FROM_SCRATCH) ld_site(s, scratch + (size_t)cg_half(g, n) * 12);
-    else ld_site(s, psi + cg_full(g, n) * 12);
-    ld_link(u, links + (self * 4 + mu) * 9);
-    // forward: U(x) (1 - isign gamma) psi(x+mu)
-    switch (mu) {
-      case 0: project<0, DAG ? 1 : -1>(h, s); break;
-      case 1: project<1, DAG ? 1 : -1>(h, s); break;
-      case 2: project<2, DAG ? 1 : -1>(h, s); break;
-      default: project<3, DAG ? 1 : -1>(h, s); break;
-    }
-    mat_vec2(uh, u, h);
-    switch (mu) {
-      case 0: reconstruct<0, DAG ? 1 : -1>(acc, uh); break;
-      case 1: reconstruct<1, DAG ? 1 : -1>(acc, uh); break;
-      case 2: reconstruct<2, DAG ? 1 : -1>(acc, uh); break;
-      default: reconstruct<3, DAG ? 1 : -1>(acc, uh); break;
-    }
-    n.x[mu] = c.x[mu] == 0 ? g.L[mu] - 1 : c.x[mu] - 1;
-    const long nb = cg_full(g, n);
-    if (FROM_SCRATCH) ld_site(s, scratch + (size_t)cg_half(g, n) * 12);
-    else ld_site(s, psi + nb * 12);
-    ld_link(u, links + (nb * 4 + mu) * 9);
-    // backward: U^dag(x-mu) (1 + isign gamma) psi(x-mu)
-    switch (mu) {
-      case 0: project<0, DAG ? -1 : 1>(h, s); break;
-      case 1: project<1, DAG ? -1 : 1>(h, s); break;
-      case 2: project<2, DAG ? -1 : 1>(h, s); break;
-      default: project<3, DAG ? -1 : 1>(h, s); break;
-    }
-    adj_mat_vec2(uh, u, h);
-    switch (mu) {
-      case 0: reconstruct<0, DAG ? -1 : 1>(acc, uh); break;
-      case 1: reconstruct<1, DAG ? -1 : 1>(acc, uh); break;
-      case 2: reconstruct<2, DAG ? -1 : 1>(acc, uh); break;
-      default: reconstruct<3, DAG ? -1 : 1>(acc, uh); break;
-    }
-  }
-}
-
 // even sites: scratch[cb] = A_ee^-1 D'_eo psi_o
-template <bool DAG>
-__global__ void noalloc_even(CanonGeom g, const double2* links, const double* invclov, const double2* psi,
-                             double2* scratch) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.Vh) return;
-  const Coord c = cg_coords(g, i, 0);
-  cplx<double> acc[12], y[12];
-  hop_canon<DAG, false>(acc, g, c, links, psi, nullptr);
-  clover_site(y, invclov + cg_full(g, c) * 72, acc);
-#pragma unroll
-  for (int k = 0; k < 12; ++k) scratch[(size_t)i * 12 + k] = make_double2(y[k].re, y[k].im);
+template <bool DAG, int S>
+__global__ void __launch_bounds__(8 * S) noalloc_even(const CanonField<0> f) {
+  double sum[3];
+  split_site<CanonField<0>, HOP_CLOV, DAG, RED_NONE, S>(f, 1.0, 0.0, blockIdx.x, sum);
 }
 
 // odd sites: out = A_oo psi_o - 1/4 D'_oe scratch  (+ isign i mu gamma_5 psi_o)
+template <bool DAG, int S>
+__global__ void __launch_bounds__(8 * S) noalloc_odd(const CanonField<1> f, double twist) {
+  double sum[3];
+  split_site<CanonField<1>, HOP_XPAY, DAG, RED_NONE, S>(f, -0.25, twist, blockIdx.x, sum);
+}
+
+template <bool DAG, int S>
+void noalloc_launch(const CanonField<0>& fe, const CanonField<1>& fo, double twist, cudaStream_t s) {
+  const unsigned blocks = (unsigned)((fe.g.Vh + S - 1) / S);
+  noalloc_even<DAG, S><<<blocks, 8 * S, 0, s>>>(fe);
+  noalloc_odd<DAG, S><<<blocks, 8 * S, 0, s>>>(fo, twist);
+}
 template <bool DAG>
-__global__ void noalloc_odd(CanonGeom g, const double2* links, const double* clov, const double2* psi,
-                            const double2* scratch, double twist, double2* out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= g.Vh) return;
-  const Coord c = cg_coords(g, i, 1);
-  const long s = cg_full(g, c);
-  cplx<double> acc[12], x[12], y[12];
-  hop_canon<DAG, true>(acc, g, c, links, nullptr, scratch);
-  ld_site(x, psi + s * 12);
-  clover_site(y, clov + s * 72, x);
-  const double tw = DAG ? -twist : twist;
-#pragma unroll
-  for (int k = 0; k < 12; ++k) {
-    cplx<double> v = y[k];
-    v.re = fmadd(-0.25, acc[k].re, v.re);
-    v.im = fmadd(-0.25, acc[k].im, v.im);
-    if (twist != 0.0) v = v + (k < 6 ? tw : -tw) * timesI(x[k]);
-    out[s * 12 + k] = make_double2(v.re, v.im);
+void noalloc_launch(const CanonField<0>& fe, const CanonField<1>& fo, double twist, cudaStream_t s) {
+  switch (hop_split_sites(fe.g.Vh, 1)) {
+    case 8: return noalloc_launch<DAG, 8>(fe, fo, twist, s);
+    case 16: return noalloc_launch<DAG, 16>(fe, fo, twist, s);
+    default: return noalloc_launch<DAG, 32>(fe, fo, twist, s);
   }
 }
 
@@ -223,7 +143,7 @@ extern "C" int gbc_apply_meo_noalloc(const gbc_geom* geom, const gbc_action* act
   double2* scratch = nullptr;
   int rc = noalloc_scratch_for_current_device(&scratch);
   if (rc != GBC_OK) return rc;
-  CanonGeom g;
+  Geom g{};
   for (int m = 0; m < 4; ++m) g.L[m] = geom->dims[m];
   g.Lxh = g.L[0] / 2;
   g.Vh = (int)(V / 2);
@@ -232,15 +152,10 @@ extern "C" int gbc_apply_meo_noalloc(const gbc_geom* geom, const gbc_action* act
   const double2* in = reinterpret_cast<const double2*>(in_dev);
   double2* out = reinterpret_cast<double2*>(out_dev);
   const double twist = act->twisted ? act->twisted_m : 0.0;
-  const int threads = 128;
-  const unsigned blocks = (unsigned)((g.Vh + threads - 1) / threads);
   // the scratch is fully overwritten by the first kernel on every call: nothing to clear
-  if (isign > 0) {
-    noalloc_even<false><<<blocks, threads, 0, s>>>(g, links, invclov_dev, in, scratch);
-    noalloc_odd<false><<<blocks, threads, 0, s>>>(g, links, clov_dev, in, scratch, twist, out);
-  } else {
-    noalloc_even<true><<<blocks, threads, 0, s>>>(g, links, invclov_dev, in, scratch);
-    noalloc_odd<true><<<blocks, threads, 0, s>>>(g, links, clov_dev, in, scratch, twist, out);
-  }
+  const CanonField<0> fe{g, links, invclov_dev, in, scratch, nullptr};
+  const CanonField<1> fo{g, links, clov_dev, in, scratch, out};
+  if (isign > 0) noalloc_launch<false>(fe, fo, twist, s);
+  else noalloc_launch<true>(fe, fo, twist, s);
   return cudaGetLastError() == cudaSuccess ? GBC_OK : GBC_ERR_CUDA;
 }
