@@ -22,26 +22,13 @@
 
 #include "ctx.h"
 #include "gbc_device.cuh"
+#include "reduce.cuh"
 
 namespace gbc {
-
-struct BiScal {
-  double2 rho, alpha, omega, beta;
-  double rr, rsd_sq;
-  int active, iters, status;
-};
 
 namespace {
 
 constexpr int BT = 256;
-
-__device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
-  const double d = b.x * b.x + b.y * b.y;
-  return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
-}
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
 
 template <typename P>
 __device__ __forceinline__ void ldv(cplx<typename P::real> (&x)[12], const Spinor& f, int idx, int r) {
@@ -111,7 +98,7 @@ __device__ __forceinline__ float site_norm(const Spinor& f, int idx, int r) {
 // its partial rows are never read.
 template <int NRED, class F>
 __global__ void __launch_bounds__(BT, F::kMinb) bi_site_kernel(int Vh, F f, const BiScal* sc, double* partials,
-                                                               int part_stride, int nrhs) {
+                                                               int part_stride, int nrhs, Finish fin) {
   using A = typename AccOf<F>::type;  // thread and warp sums in the compute precision
   const int r = blockIdx.y;
   if (!sc[r].active) return;  // uniform over the block
@@ -135,6 +122,7 @@ __global__ void __launch_bounds__(BT, F::kMinb) bi_site_kernel(int Vh, F f, cons
       for (int w = 0; w < BT / 32; ++w) s += sh[threadIdx.x][w];
       partials[((size_t)threadIdx.x * nrhs + r) * part_stride + blockIdx.x] = s;
     }
+    finish_reduction<NRED, BT>(fin, partials, part_stride, nrhs, r, gridDim.x);
   }
 }
 
@@ -250,100 +238,44 @@ struct PUpdF {
   }
 };
 
-// alpha = rho / (r0, v)          res = [Re, Im][n]
-__global__ void bi_alpha(BiScal* sc, const double* res, int n) {
-  const int k = threadIdx.x;
-  if (k >= n) return;
-  BiScal q = sc[k];
-  q.alpha = make_double2(0.0, 0.0);
-  if (q.active) {
-    const double2 d = make_double2(res[k], res[n + k]);
-    if (d.x * d.x + d.y * d.y > 0.0 && std::isfinite(d.x) && std::isfinite(d.y)) {
-      q.alpha = cdiv(q.rho, d);
-    } else {
-      q.active = 0;
-      q.status = GBC_ERR_BREAKDOWN;
-    }
-  }
-  sc[k] = q;
-}
-
-// omega = (t, s) / (t, t)         res = [Re ts, Im ts, tt][n]
-__global__ void bi_omega(BiScal* sc, const double* res, int n) {
-  const int k = threadIdx.x;
-  if (k >= n) return;
-  BiScal q = sc[k];
-  const double tt = res[2 * n + k];
-  q.omega = (q.active && tt > 0.0) ? make_double2(res[k] / tt, res[n + k] / tt) : make_double2(0.0, 0.0);
-  sc[k] = q;
-}
-
-// |r|^2, rho' = (r0, r); converged -> inactive; beta = (rho'/rho)(alpha/omega)   res = [rr, Re, Im][n]
-__global__ void bi_beta(BiScal* sc, const double* res, int n) {
-  const int k = threadIdx.x;
-  if (k >= n) return;
-  BiScal q = sc[k];
-  q.beta = make_double2(0.0, 0.0);
-  if (q.active) {
-    q.iters += 1;
-    q.rr = res[k];
-    const double2 rho1 = make_double2(res[n + k], res[2 * n + k]);
-    if (!std::isfinite(q.rr)) {
-      q.active = 0;
-      q.status = GBC_ERR_NONFINITE;
-    } else if (!(q.rr > q.rsd_sq)) {
-      q.active = 0;  // converged
-    } else if (q.omega.x == 0.0 && q.omega.y == 0.0) {
-      q.active = 0;
-      q.status = GBC_ERR_BREAKDOWN;
-    } else {
-      q.beta = cmul(cdiv(rho1, q.rho), cdiv(q.alpha, q.omega));
-    }
-    q.rho = rho1;
-  }
-  sc[k] = q;
-}
-
 template <int NRED, class F>
-void run(gbc_ctx* c, int nrhs, const BiScal* sc, const F& f) {
+void run(gbc_ctx* c, int nrhs, const BiScal* sc, const F& f, const Red& rd) {
   const Geom& g = c->g;
   dim3 grid(blas_blocks(g), nrhs);
-  const Red rd = red(c);
-  bi_site_kernel<NRED, F><<<grid, BT, 0, c->stream>>>(g.Vh, f, sc, rd.partials, rd.part_stride, nrhs);
+  const bool inside = NRED > 0 && rd.count && finish_in_kernel((long)grid.x * nrhs);
+  bi_site_kernel<NRED, F><<<grid, BT, 0, c->stream>>>(g.Vh, f, sc, rd.partials, rd.part_stride, nrhs,
+                                                      inside ? rd.finish() : Finish{});
   count_launch();
-  if (NRED > 0) reduce_finalize(rd, NRED, nrhs, grid.x, c->stream);
+  if (NRED > 0 && !inside) reduce_finalize(rd, NRED, nrhs, grid.x, c->stream);
 }
 
 template <typename PA, typename PO>
 void iteration(gbc_ctx* c, int po, BiScal* sc, int n, const Spinor& x, const Spinor& r, const Spinor& r0,
                const Spinor& p, const Spinor& v, const Spinor& s, const Spinor& t, const Spinor& te) {
-  cudaStream_t st = c->stream;
-  const int nth = ((n + 31) / 32) * 32;  // one thread per right-hand side
+  const Red rd = red(c);
+  // alpha from (r0, v)
+  const Red alpha = rd.then(FIN_BI_ALPHA, sc);
   if (!c->sym && r0.prec == PREC_SINGLE) {
     // (r0, v) summed in the epilogue of the stencil launch that writes v = M~ p (r0 at its sites)
     c->hop_aux = r0;
-    apply_meo(c, po, false, p, v, te, RED_DOT_AUX);
+    apply_meo(c, po, false, p, v, te, RED_DOT_AUX, &alpha);
     c->hop_aux = Spinor{};
   } else {
     apply_meo(c, po, false, p, v, te, RED_NONE);
-    blas_cdot(c->g, r0, v, red(c), st);
+    blas_cdot(c->g, r0, v, alpha, c->stream);
   }
-  bi_alpha<<<1, nth, 0, st>>>(sc, c->d_result, n);
-  count_launch();
-  run<0>(c, n, sc, SUpdF<PA, PO>{sc, r, v, s});
+  run<0>(c, n, sc, SUpdF<PA, PO>{sc, r, v, s}, rd);
+  // omega from (t, s) and (t, t)
+  const Red omega = rd.then(FIN_BI_OMEGA, sc);
   if (c->sym) {
     apply_meo(c, po, false, s, t, te, RED_NONE);
-    run<3>(c, n, sc, TsTtF<PO>{t, s});
+    run<3>(c, n, sc, TsTtF<PO>{t, s}, omega);
   } else {
-    // (t, s) and (t, t) summed in the epilogue of the stencil launch that writes t (s is its self)
-    apply_meo(c, po, false, s, t, te, RED_DOT_SELF);
+    // both summed in the epilogue of the stencil launch that writes t (s is its self)
+    apply_meo(c, po, false, s, t, te, RED_DOT_SELF, &omega);
   }
-  bi_omega<<<1, nth, 0, st>>>(sc, c->d_result, n);
-  count_launch();
-  run<3>(c, n, sc, XRUpdF<PA, PO>{sc, x, r, p, v, t, r0});
-  bi_beta<<<1, nth, 0, st>>>(sc, c->d_result, n);
-  count_launch();
-  run<0>(c, n, sc, PUpdF<PA, PO>{sc, r, p, v});
+  run<3>(c, n, sc, XRUpdF<PA, PO>{sc, x, r, p, v, t, r0}, rd.then(FIN_BI_BETA, sc));
+  run<0>(c, n, sc, PUpdF<PA, PO>{sc, r, p, v}, rd);
 }
 
 }  // namespace
@@ -368,9 +300,9 @@ void bicgstab_xr_update(gbc_ctx* c, int pa, int po, const double* alpha_omega, i
     hs[i].active = 1;
   }
   GBC_CUDA(cudaMemcpyAsync(d_sc, hs.data(), sizeof(BiScal) * n, cudaMemcpyHostToDevice, c->stream));
-  if (pa == PREC_DOUBLE) run<3>(c, n, d_sc, XRUpdF<PrecD, PrecD>{d_sc, x, r, p, v, t, r0});
-  else if (po == PREC_SINGLE) run<3>(c, n, d_sc, XRUpdF<PrecS, PrecS>{d_sc, x, r, p, v, t, r0});
-  else run<3>(c, n, d_sc, XRUpdF<PrecS, PrecH>{d_sc, x, r, p, v, t, r0});
+  if (pa == PREC_DOUBLE) run<3>(c, n, d_sc, XRUpdF<PrecD, PrecD>{d_sc, x, r, p, v, t, r0}, red(c));
+  else if (po == PREC_SINGLE) run<3>(c, n, d_sc, XRUpdF<PrecS, PrecS>{d_sc, x, r, p, v, t, r0}, red(c));
+  else run<3>(c, n, d_sc, XRUpdF<PrecS, PrecH>{d_sc, x, r, p, v, t, r0}, red(c));
   GBC_CUDA(cudaGetLastError());
   sync(c);  // hs goes out of scope
 }

@@ -1,11 +1,13 @@
 // BLAS-1 on checkerboard spinor fields (any storage precision per operand).  Reductions sum a
 // thread's sites and a warp's lanes in the operands' compute precision (FP32 unless an operand is
 // FP64: GB300's FP64 pipe made per-site FP64 sums the bottleneck of bandwidth-bound kernels), then
-// per-warp and per-block sums in FP64 in a fixed grid, then one deterministic finalize pass.  Also the device-side CG scalar logic, so that an iteration
-// needs no host round trip (InvCG2, lib/actions/ferm/invert/invcg2.cc:153-221).
+// per-warp and per-block sums in FP64 in a fixed grid; the last block sums the partials in a fixed
+// order and applies the solver's scalar step (reduce.cuh), so that an iteration needs no host round
+// trip (InvCG2, lib/actions/ferm/invert/invcg2.cc:153-221).
 #include <string>
 
 #include "gbc_device.cuh"
+#include "reduce.cuh"
 
 namespace gbc {
 
@@ -15,7 +17,8 @@ constexpr int BLAS_THREADS = 256;
 
 // grid-stride driver: f(idx, rhs, acc) per site; NRED doubles reduced per right-hand side
 template <int NRED, class F>
-__global__ void __launch_bounds__(BLAS_THREADS) site_kernel(int Vh, F f, double* partials, int part_stride, int nrhs) {
+__global__ void __launch_bounds__(BLAS_THREADS) site_kernel(int Vh, F f, double* partials, int part_stride, int nrhs,
+                                                            Finish fin) {
   using A = typename AccOf<F>::type;
   const int r = blockIdx.y;
   A acc[NRED > 0 ? NRED : 1];
@@ -38,6 +41,7 @@ __global__ void __launch_bounds__(BLAS_THREADS) site_kernel(int Vh, F f, double*
       for (int w = 0; w < BLAS_THREADS / 32; ++w) s += sh[threadIdx.x][w];
       partials[((size_t)threadIdx.x * nrhs + r) * part_stride + blockIdx.x] = s;
     }
+    finish_reduction<NRED, BLAS_THREADS>(fin, partials, part_stride, nrhs, r, gridDim.x);
   }
 }
 
@@ -329,41 +333,22 @@ __global__ void finalize_kernel(const double* partials, int part_stride, int nbl
   if (threadIdx.x == 0) result[qr] = sh[0];
 }
 
-__global__ void cg_alpha_kernel(CGScalars* st, const double* red_d, double* a_out, int nrhs) {
-  const int r = threadIdx.x;
-  if (r >= nrhs) return;
-  CGScalars s = st[r];
-  s.d = red_d[r];
-  s.a = (s.active && s.d > 0.0) ? s.c / s.d : 0.0;
-  a_out[r] = s.a;
-  st[r] = s;
-}
-
-__global__ void cg_beta_kernel(CGScalars* st, const double* red_r, double* b_out, int nrhs) {
-  const int r = threadIdx.x;
-  if (r >= nrhs) return;
-  CGScalars s = st[r];
-  if (s.active) {
-    s.cp = red_r[r];
-    s.iters += 1;
-    if (!(s.cp > s.rsd_sq)) s.active = 0;  // converged (or non-finite: stops and is reported)
-    s.b = (s.active && s.c > 0.0) ? s.cp / s.c : 0.0;
-    s.c_prev = s.c;
-    s.c = s.cp;
-  } else {
-    s.b = 0.0;
-  }
-  b_out[r] = s.b;
-  st[r] = s;
+// the sums of one right-hand side per block, and their scalar step
+template <int NQ>
+__global__ void __launch_bounds__(256) finish_kernel(Finish f, const double* partials, int part_stride, int nrhs,
+                                                     int nblocks) {
+  sum_partials<NQ, 256>(f, partials, part_stride, nrhs, blockIdx.x, nblocks);
 }
 
 template <int NRED, class F>
 void run(const Geom& g, int nrhs, const F& f, const Red* red, cudaStream_t s) {
   dim3 grid(blas_blocks(g), nrhs);
+  const bool inside = NRED > 0 && red->count && finish_in_kernel((long)grid.x * nrhs);
   site_kernel<NRED, F><<<grid, BLAS_THREADS, 0, s>>>(g.Vh, f, red ? red->partials : nullptr,
-                                                     red ? red->part_stride : 0, nrhs);
+                                                     red ? red->part_stride : 0, nrhs,
+                                                     inside ? red->finish() : Finish{});
   count_launch();
-  if (NRED > 0) reduce_finalize(*red, NRED, nrhs, grid.x, s);
+  if (NRED > 0 && !inside) reduce_finalize(*red, NRED, nrhs, grid.x, s);
 }
 
 }  // namespace
@@ -376,7 +361,10 @@ int blas_blocks(const Geom& g) {
 }
 
 void reduce_finalize(const Red& red, int nred, int nrhs, int nblocks, cudaStream_t s) {
-  finalize_kernel<<<nred * nrhs, 256, 0, s>>>(red.partials, red.part_stride, nblocks, red.result);
+  if (red.kind == FIN_SUM) finalize_kernel<<<nred * nrhs, 256, 0, s>>>(red.partials, red.part_stride, nblocks, red.result);
+  else if (nred == 1) finish_kernel<1><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
+  else if (nred == 2) finish_kernel<2><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
+  else finish_kernel<3><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
   count_launch();
 }
 
@@ -443,15 +431,6 @@ void blas_xpy(const Geom& g, const Spinor& x, const Spinor& y, cudaStream_t s) {
 }
 void blas_xsub_norm2(const Geom& g, const Spinor& x, const Spinor& y, const Red& red, cudaStream_t s) {
   GBC_DISPATCH2(x.prec, y.prec, (run<1>(g, x.nrhs, XsubNormF<PA, PB>{x, y}, &red, s)));
-}
-
-void cg_alpha(CGScalars* st, const double* red_d, double* a_out, int nrhs, cudaStream_t s) {
-  cg_alpha_kernel<<<1, 32, 0, s>>>(st, red_d, a_out, nrhs);
-  count_launch();
-}
-void cg_beta(CGScalars* st, const double* red_r, double* b_out, int nrhs, cudaStream_t s) {
-  cg_beta_kernel<<<1, 32, 0, s>>>(st, red_r, b_out, nrhs);
-  count_launch();
 }
 
 }  // namespace gbc

@@ -66,7 +66,7 @@ Spinor sub(const Spinor& s, int r0, int n) {
   return t;
 }
 
-Red red(gbc_ctx* c) { return Red{c->d_partials, c->part_stride, c->d_result}; }
+Red red(gbc_ctx* c) { return Red{c->d_partials, c->part_stride, c->d_result, c->d_count}; }
 
 void ensure_stage(gbc_ctx* c, int nrhs) {
   size_t need = (size_t)nrhs * c->V * 24;
@@ -172,6 +172,7 @@ void free_ctx_memory(gbc_ctx* c) {
   if (c->d_ca) cudaFree(c->d_ca);
   if (c->d_cb) cudaFree(c->d_cb);
   if (c->d_cg) cudaFree(c->d_cg);
+  if (c->d_count) cudaFree(c->d_count);
   for (int i = 0; i < 2; ++i)
     if (c->d_stage[i]) cudaFree(c->d_stage[i]);
   if (c->d_kpartials) cudaFree(c->d_kpartials);
@@ -393,7 +394,7 @@ static Spinor split_copy(gbc_ctx* c, int slot, const Spinor& x) {
 }
 
 void hop(gbc_ctx* c, int prec, int out_parity, int mode, bool dag, double a, const Spinor& in_field,
-         const Spinor& out, const Spinor* self, const void* clov, int reduce, double twist) {
+         const Spinor& out, const Spinor* self, const void* clov, int reduce, double twist, const Red* rd) {
   const PrecFields& f = c->pf[pidx(prec)];
   Spinor in = in_field, self_split;
   if (prec == PREC_DF) {
@@ -435,26 +436,37 @@ void hop(gbc_ctx* c, int prec, int out_parity, int mode, bool dag, double a, con
     h.aux = c->hop_aux.v;
     h.aux_rhs_bytes = c->hop_aux.rhs_bytes;
   }
+  const Red sums = rd ? *rd : red(c);
   int nb;
+  bool finished = false;  // the kernel ends its reduction itself
+  // (the autotuner's launches above carry no finish: they would repeat the scalar step)
+  const auto set_finish = [&](int blocks, bool one_rhs) {
+    finished = reduce && one_rhs && finish_in_kernel((long)blocks * h.nrhs);
+    if (finished) h.fin = sums.finish();
+  };
   if (prec == PREC_DOUBLE && hop_split(h.g.Vh, h.nrhs)) {
-    nb = hop_split_launch(mode, dag, reduce, h, hop_split_sites(h.g.Vh, h.nrhs), c->stream);
+    const int sites = hop_split_sites(h.g.Vh, h.nrhs);
+    set_finish((h.g.Vh + sites - 1) / sites, true);
+    nb = hop_split_launch(mode, dag, reduce, h, sites, c->stream);
   } else {
     const HopShape sh = kHopShapes[tuned_shape(c, prec, f.recon, mode, dag, reduce, h)];
     if (hop_blocks(sh, h.g.Vh) > c->part_stride) throw std::string("partials buffer too small");
+    set_finish(hop_blocks(sh, h.g.Vh), sh.nrb == 1);
     nb = hop_launch(prec, f.recon, mode, dag, reduce, h, sh, c->stream);
   }
   if (nb < 0) throw std::string("hopping kernel variant not compiled");
   count_launch();
   GBC_CUDA(cudaGetLastError());
-  if (reduce) reduce_finalize(red(c), red_rows(reduce), in.nrhs, nb, c->stream);
+  if (reduce && !finished) reduce_finalize(sums, red_rows(reduce), in.nrhs, nb, c->stream);
 }
 
-void apply_meo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce) {
-  if (c->sym) return apply_seo(c, prec, dag, in, out, tmp_e, reduce);
+void apply_meo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce,
+               const Red* rd) {
+  if (c->sym) return apply_seo(c, prec, dag, in, out, tmp_e, reduce, rd);
   const PrecFields& f = c->pf[pidx(prec)];
   // t_e = A_ee^-1 D_eo in_o ;  out_o = A_oo in_o - 1/4 D_oe t_e  (+ isign i mu gamma_5 in_o)
   hop(c, prec, 0, HOP_CLOV, dag, 1.0, in, tmp_e, nullptr, f.clovinv, false);
-  hop(c, prec, 1, HOP_XPAY, dag, -0.25, tmp_e, out, &in, f.clov[1], reduce, c->act.twisted ? c->act.twisted_m : 0.0);
+  hop(c, prec, 1, HOP_XPAY, dag, -0.25, tmp_e, out, &in, f.clov[1], reduce, c->act.twisted ? c->act.twisted_m : 0.0, rd);
 }
 
 void apply_clover(gbc_ctx* c, int prec, int parity, bool inverse, const Spinor& in, const Spinor& out) {
@@ -490,7 +502,7 @@ void ensure_sym(gbc_ctx* c, int prec) {
 // with a twisted-mass term, in - out + isign i mu gamma_5 in (seoprec_clover_linop_w.cc:174-184:
 // the clover term and its inverses carry no twist, the term is added to M_s itself).
 void apply_seo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e,
-               int reduce) {
+               int reduce, const Red* rd) {
   ensure_sym(c, prec);
   const PrecFields& f = c->pf[pidx(prec)];
   if (!dag) {
@@ -502,10 +514,11 @@ void apply_seo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& o
     hop(c, prec, 0, HOP_CLOV, true, 1.0, to, tmp_e, nullptr, f.clovinv, false);
     hop(c, prec, 1, HOP_PLAIN, true, 0.25, tmp_e, out, nullptr, nullptr, false);
   }
+  const Red sums = rd ? *rd : red(c);
   if (c->act.twisted && c->act.twisted_m != 0.0)
-    blas_xmy_twist_norm2(c->g, in, out, dag ? -c->act.twisted_m : c->act.twisted_m, red(c), c->stream);
+    blas_xmy_twist_norm2(c->g, in, out, dag ? -c->act.twisted_m : c->act.twisted_m, sums, c->stream);
   else
-    blas_xmy_norm2(c->g, in, out, red(c), c->stream);
+    blas_xmy_norm2(c->g, in, out, sums, c->stream);
   (void)reduce;
 }
 
@@ -606,6 +619,8 @@ int gbc_create(gbc_ctx** out, const gbc_geom* geom, const gbc_action* act, const
     GBC_CUDA(cudaMalloc(&c->d_partials, sizeof(double) * 3 * c->max_rhs * (size_t)c->part_stride));
     GBC_CUDA(cudaMalloc(&c->d_result, sizeof(double) * 3 * c->max_rhs));
     GBC_CUDA(cudaMallocHost(&c->h_result, sizeof(double) * 3 * c->max_rhs));
+    GBC_CUDA(cudaMalloc(&c->d_count, sizeof(unsigned) * 4 * c->max_rhs));
+    GBC_CUDA(cudaMemset(c->d_count, 0, sizeof(unsigned) * 4 * c->max_rhs));
     GBC_CUDA(cudaMalloc(&c->d_cg, sizeof(CGScalars) * c->max_rhs));
     GBC_CUDA(cudaMallocHost(&c->h_cg, sizeof(CGScalars) * c->max_rhs));
     GBC_CUDA(cudaMalloc(&c->d_a, sizeof(double) * c->max_rhs));

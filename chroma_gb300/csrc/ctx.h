@@ -67,6 +67,7 @@ struct gbc_ctx {
   int part_stride = 0;
   double* d_partials = nullptr;
   double* d_result = nullptr;
+  unsigned* d_count = nullptr;  // arrival counters of the reductions, one per right-hand side
   double* h_result = nullptr;  // pinned
   gbc::CGScalars* d_cg = nullptr;
   gbc::CGScalars* h_cg = nullptr;  // pinned
@@ -128,12 +129,14 @@ Red red(gbc_ctx* c);
 // ---- operator blocks on device fields (all of precision prec) ------------------------------
 // out(out_parity) = mode-epilogue of a * D'(in)
 void hop(gbc_ctx* c, int prec, int out_parity, int mode, bool dag, double a, const Spinor& in, const Spinor& out,
-         const Spinor* self, const void* clov, int reduce, double twist = 0.0);
-// out_o = M~ in_o (dag: M~^dag); reduce => |out|^2 in red(c).result[0][rhs]
-void apply_meo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce);
+         const Spinor* self, const void* clov, int reduce, double twist = 0.0, const Red* rd = nullptr);
+// out_o = M~ in_o (dag: M~^dag); reduce => |out|^2 in red(c).result[0][rhs]; rd: red(c) with a scalar step
+void apply_meo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce,
+               const Red* rd = nullptr);
 void apply_clover(gbc_ctx* c, int prec, int parity, bool inverse, const Spinor& in, const Spinor& out);
 // out_o = M_s in_o (dag: M_s^dag), the symmetric operator; reduce => |out|^2 as apply_meo
-void apply_seo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce);
+void apply_seo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e, int reduce,
+               const Red* rd = nullptr);
 void ensure_sym(gbc_ctx* c, int prec);  // pack A_oo^-1 in this precision
 // routes apply_meo to the symmetric operator while it lives
 struct SymScope {

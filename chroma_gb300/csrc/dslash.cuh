@@ -20,6 +20,7 @@
 #pragma once
 #include "gbc_device.cuh"
 #include "gbc_kernels.h"
+#include "reduce.cuh"
 
 namespace gbc {
 
@@ -825,13 +826,15 @@ __device__ __forceinline__ void hop_body(const HopArgs& a, int sblock, int group
         if (r < a.nrhs) a.partials[((size_t)q * a.nrhs + r) * a.part_stride + sblock] = s;
       }
     }
+    if constexpr (NRB == 1)
+      finish_reduction<NQ, TX>(a.fin, a.partials, a.part_stride, a.nrhs, group, (g.Vh + TX - 1) / TX);
   }
 }
 
-// block sums of a one-right-hand-side block of NT threads (pair and ring kernels): partial rows
-// q * nrhs + rhs
+// block sums of a one-right-hand-side block of NT threads (pair, ring and split kernels): partial
+// rows q * nrhs + rhs; nblk blocks of the right-hand side
 template <int NQ, int NT, typename T>
-__device__ __forceinline__ void block_sums_1rhs(const HopArgs& a, Sums3<T> local, int rhs, int sblock) {
+__device__ __forceinline__ void block_sums_1rhs(const HopArgs& a, Sums3<T> local, int rhs, int sblock, int nblk) {
   __shared__ double wsum[NQ][NT / 32];
 #pragma unroll
   for (int q = 0; q < NQ; ++q) {
@@ -848,6 +851,7 @@ __device__ __forceinline__ void block_sums_1rhs(const HopArgs& a, Sums3<T> local
     for (int w = 0; w < NT / 32; ++w) s += wsum[q][w];
     a.partials[((size_t)q * a.nrhs + rhs) * a.part_stride + sblock] = s;
   }
+  finish_reduction<NQ, NT>(a.fin, a.partials, a.part_stride, a.nrhs, rhs, nblk);
 }
 
 // ---- fp16 storage, two sites per thread ---------------------------------------------------------
@@ -1062,7 +1066,7 @@ __global__ void __launch_bounds__(TX, MINB) hop_kernel_pair(const HopArgs a) {
     }
     local = hop_epilogue<PrecH, MODE, DAG, REDUCE>(a, rhs, ia, sa) + hop_epilogue<PrecH, MODE, DAG, REDUCE>(a, rhs, ib, sb);
   }
-  if constexpr (REDUCE != RED_NONE) block_sums_1rhs<red_count<REDUCE>(), TX>(a, local, rhs, sblock);
+  if constexpr (REDUCE != RED_NONE) block_sums_1rhs<red_count<REDUCE>(), TX>(a, local, rhs, sblock, (half + TX - 1) / TX);
 }
 
 }  // namespace gbc

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(TX, MINB) hop_kernel_async(const HopArgs a) {
     for (int k = 0; k < 12; ++k) out[k] = {acc[k].x, acc[k].y};
     local = hop_epilogue<PrecH, MODE, DAG, REDUCE>(a, rhs, idx, out);
   }
-  if constexpr (REDUCE != RED_NONE) block_sums_1rhs<red_count<REDUCE>(), TX>(a, local, rhs, sblock);
+  if constexpr (REDUCE != RED_NONE) block_sums_1rhs<red_count<REDUCE>(), TX>(a, local, rhs, sblock, (g.Vh + TX - 1) / TX);
 }
 
 }  // namespace gbc

@@ -13,7 +13,8 @@ __global__ void __launch_bounds__(8 * S) hop_kernel_split(const HopArgs a) {
   if (!a.active || a.active[(size_t)rhs * a.active_stride])
     split_site<SplitPlanes, MODE, DAG, REDUCE, S>(SplitPlanes{a, rhs}, a.a, a.twist, sblock, sum);
   if constexpr (REDUCE != RED_NONE)
-    block_sums_1rhs<red_count<REDUCE>(), 8 * S>(a, Sums3<double>{{sum[0], sum[1], sum[2]}}, rhs, sblock);
+    block_sums_1rhs<red_count<REDUCE>(), 8 * S>(a, Sums3<double>{{sum[0], sum[1], sum[2]}}, rhs, sblock,
+                                                (a.g.Vh + S - 1) / S);
 }
 
 template <int MODE, bool DAG, int REDUCE>

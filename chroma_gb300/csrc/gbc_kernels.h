@@ -21,6 +21,34 @@ enum { PREC_HALF = 2, PREC_SINGLE = 4, PREC_DOUBLE = 8 };
 // (the PrecDF kernels on the split copies of the FP64 links and clover)
 enum { PREC_DF = 16 };
 
+// device scalars of the solvers, one per right-hand side
+struct CGScalars {
+  double c, d, a, b, cp, rsd_sq, c_prev;
+  int active, iters;
+};
+struct BiScal {
+  double2 rho, alpha, omega, beta;
+  double rr, rsd_sq;
+  int active, iters, status;
+};
+
+// What happens to a reduction's finished sums (reduce.cuh): nothing inside the kernel; the sums
+// into result; or also the scalar step of CG (CGScalars, alpha or beta into coef) or BiCGStab (BiScal).
+enum { FIN_NONE = 0, FIN_SUM, FIN_CG_ALPHA, FIN_CG_BETA, FIN_BI_ALPHA, FIN_BI_OMEGA, FIN_BI_BETA };
+struct Finish {
+  int kind = FIN_NONE;
+  unsigned* count = nullptr;  // arrived blocks per right-hand side, zero between launches
+  double* result = nullptr;   // [quantity][rhs]
+  void* sc = nullptr;         // CGScalars or BiScal per right-hand side
+  double* coef = nullptr;     // CG: alpha or beta per right-hand side
+};
+// Where a reduction ends inside its kernel: grids of up to about one resident wave.  Each block then stays
+// about 1 us longer (its arrival is an atomic whose answer it needs), which costs nothing while no
+// block waits for its place: FP64 CG on 8^3 x 16, 40 iterations.  On a 12-right-hand-side solve at
+// 16^3 x 32 (3072 and more blocks a launch) it cost 2 % against a launch of one block per right-hand
+// side, finish_kernel, which larger grids and blocks of several right-hand sides use.
+inline bool finish_in_kernel(long nblocks) { return nblocks <= 152 * 8; }
+
 struct Geom {
   int L[4];
   int Lxh;
@@ -68,6 +96,7 @@ struct HopArgs {
   // RED_DOT_AUX: the FP32 field (per right-hand side, planes of stride g.stride) dotted with out
   const void* aux;
   size_t aux_rhs_bytes;
+  Finish fin;  // end of the reduction, in kernels with one right-hand side per block
 };
 
 // Launch geometry chosen by the caller (autotuned): TX sites x NRB right-hand sides per block,
@@ -186,6 +215,18 @@ struct Red {
   double* partials;  // [nred][nrhs][part_stride]
   int part_stride;
   double* result;    // [nred][nrhs]
+  unsigned* count = nullptr;  // arrival counters (Finish); nullptr: the sums take a launch of their own
+  int kind = FIN_SUM;         // scalar step on the sums, its scalars and coefficients
+  void* sc = nullptr;
+  double* coef = nullptr;
+  Finish finish() const { return Finish{kind, count, result, sc, coef}; }
+  Red then(int kind_, void* sc_, double* coef_ = nullptr) const {
+    Red r = *this;
+    r.kind = kind_;
+    r.sc = sc_;
+    r.coef = coef_;
+    return r;
+  }
 };
 int blas_blocks(const Geom& g);  // blocks per right-hand side of the reduction kernels
 
@@ -214,18 +255,9 @@ void blas_shift_axpy(const Geom& g, const double* sigma, const Spinor& x, const 
 void blas_xpy(const Geom& g, const Spinor& x, const Spinor& y, cudaStream_t s);
 // x -= y (y may be lower precision), result = |x|^2
 void blas_xsub_norm2(const Geom& g, const Spinor& x, const Spinor& y, const Red& red, cudaStream_t s);
-// finalize the partial sums of nred quantities x nrhs into red.result
+// sum the partials of nred (any number without, at most 3 with a scalar step) quantities x nrhs into
+// red.result, then red's scalar step
 void reduce_finalize(const Red& red, int nred, int nrhs, int nblocks, cudaStream_t s);
-
-// ---- CG scalar control on the device (blas.cu) ------------------------------------------------
-struct CGScalars {
-  double c, d, a, b, cp, rsd_sq, c_prev;
-  int active, iters;
-};
-// after |M p|^2 is in red_d: d = red_d[r]; a = active ? c/d : 0
-void cg_alpha(CGScalars* st, const double* red_d, double* a_out, int nrhs, cudaStream_t s);
-// after |r|^2 is in red_r: cp; converged -> active = 0; b = active ? cp/c : 0; c = cp; iters++
-void cg_beta(CGScalars* st, const double* red_r, double* b_out, int nrhs, cudaStream_t s);
 
 // One lattice of a batched CGNE (batch_kernels.cu): its inner vectors, scalars and partial sums.
 struct LatCg {

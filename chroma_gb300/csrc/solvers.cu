@@ -133,21 +133,19 @@ CgStats cg_normal(gbc_ctx* c, const CgCfg& cfg, const Spinor& x, const Spinor& b
   blas_copy(g, p, r, s);
   bool any = false;
   for (int i = 0; i < n; ++i) any |= hs[i].active != 0;
+  const Red alpha = red(c).then(FIN_CG_ALPHA, c->d_cg, c->d_a), beta = red(c).then(FIN_CG_BETA, c->d_cg, c->d_b);
   // One iteration, all scalars on the device: no host round trip inside.
   auto body = [&]() {
     if (cfg.shift) {
       // mmp = (M~^dag M~ + shift) p and p^dag mmp -> result
       apply_meo(c, cfg.po, false, p, mp, te, false);
       apply_meo(c, cfg.po, true, mp, mmp, te, false);
-      blas_shift_dot(g, cfg.shift, p, mmp, red(c), s);
-      cg_alpha(c->d_cg, c->d_result, c->d_a, n, s);
+      blas_shift_dot(g, cfg.shift, p, mmp, alpha, s);
     } else {
-      apply_meo(c, cfg.po, false, p, mp, te, true);     // |mp|^2 -> result
-      cg_alpha(c->d_cg, c->d_result, c->d_a, n, s);
+      apply_meo(c, cfg.po, false, p, mp, te, true, &alpha);  // |mp|^2 -> result, alpha
       apply_meo(c, cfg.po, true, mp, mmp, te, false);
     }
-    blas_cg_update(g, c->d_a, x, p, r, mmp, red(c), s);  // |r|^2 -> result
-    cg_beta(c->d_cg, c->d_result, c->d_b, n, s);
+    blas_cg_update(g, c->d_a, x, p, r, mmp, beta, s);  // |r|^2 -> result, beta
     blas_xpay(g, r, c->d_b, p, s);                     // p = r + b p (b = 0 once converged)
   };
   // Blocks of kBlock iterations between host checks, replayed from a CUDA graph captured after
