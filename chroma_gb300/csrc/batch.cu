@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "ctx.h"
+#include "hostmem.h"
 
 struct gbc_batch {
   std::vector<gbc_ctx*> ctx;
@@ -158,6 +159,9 @@ int gbc_batch_solve(gbc_batch* b, const gbc_solve_params* pp, double* const* psi
       if (c->pf[pidx(sloppy)].recon != b->ctx[0]->pf[pidx(sloppy)].recon)
         throw std::string("lattices of a batch need the same link reconstruction");
     }
+    std::vector<HostResult::Item> items;
+    for (int l = 0; l < n; ++l) items.push_back({psi[l], b->ctx[l]->d_stage[1], sizeof(double) * 24 * b->ctx[l]->V});
+    HostResult out(s, copy_stream(b->ctx[0]), std::move(items), HostResult::kLoad);
     struct L {
       Spinor x, bd, rd, t1, t2, ted, rs, es, rhs, r, pv, mp, mmp, te, th1, teh;
       double bb = 0, rr = 0, prev_rr = HUGE_VAL;
@@ -432,11 +436,12 @@ int gbc_batch_solve(gbc_batch* b, const gbc_solve_params* pp, double* const* psi
     for (int l = 0; l < n; ++l) {
       gbc_ctx* c = b->ctx[l];
       L& q = lat[l];
-      GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], psi[l], sizeof(double) * 24 * c->V, cudaMemcpyHostToDevice, s));
+      out.ready();
       export_spinor(c->g, c->d_stage[1], (size_t)c->V * 24, 1, q.x, s);
-      GBC_CUDA(cudaMemcpyAsync(psi[l], c->d_stage[1], sizeof(double) * 24 * c->V, cudaMemcpyDeviceToHost, s));
+      out.send(l);
     }
     GBC_CUDA(cudaStreamSynchronize(s));
+    out.wait();
     float ms = 0;
     GBC_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     cudaEventDestroy(e0);

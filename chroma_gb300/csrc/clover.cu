@@ -118,8 +118,9 @@ __device__ void ldl_invert_block(double* d, cplx<double>* o, double& logdet, int
   for (int i = 0; i < 15; ++i) o[i] = inv_o[i];
 }
 
-__global__ void clover_build_kernel(Dims D, const double2* canon, CloverCoeffs cc, double* clov, double* inv,
-                                    double* logdet, int* nneg, int inv_parity, long V) {
+// the clover term and its inverse at the thread's site; logdet, nneg and the parity par of the site
+__device__ __forceinline__ void build_site(Dims D, const double2* canon, CloverCoeffs cc, double* clov, double* inv,
+                                    int inv_parity, long V, double& logdet, int& nneg, int& par) {
   const long s = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (s >= V) return;
   int x[4];
@@ -202,11 +203,9 @@ __global__ void clover_build_kernel(Dims D, const double2* canon, CloverCoeffs c
       out[12 + 30 * b + 2 * i + 1] = offd[b][i].im;
     }
   double* io = inv + s * 72;
-  const int par = (x[0] + x[1] + x[2] + x[3]) & 1;
+  par = (x[0] + x[1] + x[2] + x[3]) & 1;
   if (inv_parity != 2 && par != inv_parity) {
     for (int i = 0; i < 72; ++i) io[i] = 0.0;
-    logdet[s] = 0.0;
-    nneg[s] = 0;
     return;
   }
   double ld = 0.0;
@@ -219,8 +218,29 @@ __global__ void clover_build_kernel(Dims D, const double2* canon, CloverCoeffs c
       io[12 + 30 * b + 2 * i] = offd[b][i].re;
       io[12 + 30 * b + 2 * i + 1] = offd[b][i].im;
     }
-  logdet[s] = ld;
-  nneg[s] = nn;
+  logdet = ld;
+  nneg = nn;
+}
+
+constexpr int kBuildThreads = 64;
+
+// one thread per site; the block's sums of log|d| per parity and of the even sites' negative pivots
+__global__ void __launch_bounds__(kBuildThreads) clover_build_kernel(Dims D, const double2* canon, CloverCoeffs cc,
+                                                                     double* clov, double* inv, int inv_parity, long V,
+                                                                     double* sums, int sums_stride) {
+  double ld = 0.0;
+  int nn = 0, par = 0;
+  build_site(D, canon, cc, clov, inv, inv_parity, V, ld, nn, par);
+  double v[3] = {par ? 0.0 : ld, par ? ld : 0.0, par ? 0.0 : (double)nn};
+  __shared__ double sh[3][kBuildThreads / 32];
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], off);
+    if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = v[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) sums[(size_t)threadIdx.x * sums_stride + blockIdx.x] = sh[threadIdx.x][0] + sh[threadIdx.x][1];
 }
 
 __global__ void clover_invert_kernel(long n, double* packed, double* logdet, int* nneg) {
@@ -249,12 +269,14 @@ __global__ void clover_invert_kernel(long n, double* packed, double* logdet, int
 
 }  // namespace
 
-void clover_build(const int dims[4], const double* canon_links, const CloverCoeffs& cc, double* clov, double* inv,
-                  double* logdet, int* nneg, int inv_parity, cudaStream_t s) {
+int clover_build(const int dims[4], const double* canon_links, const CloverCoeffs& cc, double* clov, double* inv,
+                 double* sums, int sums_stride, int inv_parity, cudaStream_t s) {
   Dims D{{dims[0], dims[1], dims[2], dims[3]}};
   long V = (long)dims[0] * dims[1] * dims[2] * dims[3];
-  clover_build_kernel<<<(unsigned)((V + 63) / 64), 64, 0, s>>>(D, reinterpret_cast<const double2*>(canon_links), cc,
-                                                               clov, inv, logdet, nneg, inv_parity, V);
+  const int nb = (int)((V + kBuildThreads - 1) / kBuildThreads);
+  clover_build_kernel<<<nb, kBuildThreads, 0, s>>>(D, reinterpret_cast<const double2*>(canon_links), cc, clov, inv,
+                                                   inv_parity, V, sums, sums_stride);
+  return nb;
 }
 
 // inv = A^-1 on the sites of parity `parity` (clov on all sites, canonical site order)

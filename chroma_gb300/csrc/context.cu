@@ -9,6 +9,7 @@
 #include <mutex>
 
 #include "ctx.h"
+#include "hostmem.h"
 
 namespace gbc {
 
@@ -79,6 +80,11 @@ void ensure_stage(gbc_ctx* c, int nrhs) {
   c->stage_cap = need;
 }
 
+cudaStream_t copy_stream(gbc_ctx* c) {
+  if (!c->copy_stream) GBC_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
+  return c->copy_stream;
+}
+
 static size_t gauge_plane_bytes(int prec, int recon) {
   int nc = recon == 18 ? 9 : 6;
   if (prec == PREC_DOUBLE) return 16 * nc;
@@ -99,6 +105,11 @@ static void free_prec(PrecFields& f) {
   f = PrecFields{};
 }
 
+// a buffer of the packed fields: kept from one gauge field to the next
+static void take(void** p, size_t bytes) {
+  if (!*p) GBC_CUDA(cudaMalloc(p, bytes));
+}
+
 void ensure_prec(gbc_ctx* c, int prec) {
   PrecFields& f = c->pf[pidx(prec)];
   if (f.ready) return;
@@ -108,19 +119,18 @@ void ensure_prec(gbc_ctx* c, int prec) {
     // the FP64 links and clover with every double split into (hi, lo) floats, same layout
     ensure_prec(c, PREC_DOUBLE);
     const PrecFields& d = c->pf[pidx(PREC_DOUBLE)];
-    free_prec(f);
     const size_t gb = gauge_plane_bytes(PREC_DOUBLE, 18) * g.stride;
     for (int p = 0; p < 2; ++p)
       for (int m = 0; m < 4; ++m) {
-        GBC_CUDA(cudaMalloc(&f.gauge[p][m], gb));
+        take(&f.gauge[p][m], gb);
         split_df64((const double*)d.gauge[p][m], (float2*)f.gauge[p][m], gb / 8, c->stream);
       }
     const size_t cb = clover_bytes(PREC_DOUBLE) * g.stride;
     for (int p = 0; p < 2; ++p) {
-      GBC_CUDA(cudaMalloc(&f.clov[p], cb));
+      take(&f.clov[p], cb);
       split_df64((const double*)d.clov[p], (float2*)f.clov[p], cb / 8, c->stream);
     }
-    GBC_CUDA(cudaMalloc(&f.clovinv, cb));
+    take(&f.clovinv, cb);
     split_df64((const double*)d.clovinv, (float2*)f.clovinv, cb / 8, c->stream);
     GBC_CUDA(cudaGetLastError());
     sync(c);
@@ -129,13 +139,13 @@ void ensure_prec(gbc_ctx* c, int prec) {
     return;
   }
   int recon = prec == PREC_DOUBLE ? 18 : c->opts.sloppy_reconstruct;
-  float* d_err = nullptr;
-  GBC_CUDA(cudaMalloc(&d_err, sizeof(float)));
+  float* d_err = reinterpret_cast<float*>(c->d_result);  // free between solver calls
   for (int attempt = 0; attempt < 2; ++attempt) {
-    free_prec(f);
+    if (f.recon != recon) free_prec(f);  // planes of another size
+    f.recon = recon;
     size_t gb = gauge_plane_bytes(prec, recon) * g.stride;
     for (int p = 0; p < 2; ++p)
-      for (int m = 0; m < 4; ++m) GBC_CUDA(cudaMalloc(&f.gauge[p][m], gb));
+      for (int m = 0; m < 4; ++m) take(&f.gauge[p][m], gb);
     GBC_CUDA(cudaMemsetAsync(d_err, 0, sizeof(float), c->stream));
     pack_gauge(g, c->d_links, prec, recon, f.gauge, c->link_coeff, d_err, c->stream);
     float err = 0;
@@ -149,11 +159,9 @@ void ensure_prec(gbc_ctx* c, int prec) {
     }
     break;
   }
-  cudaFree(d_err);
-  f.recon = recon;
   size_t cb = clover_bytes(prec) * g.stride;
-  for (int p = 0; p < 2; ++p) GBC_CUDA(cudaMalloc(&f.clov[p], cb));
-  GBC_CUDA(cudaMalloc(&f.clovinv, cb));
+  for (int p = 0; p < 2; ++p) take(&f.clov[p], cb);
+  take(&f.clovinv, cb);
   pack_clover(g, c->d_clov, prec, f.clov, 3, c->stream);
   void* inv_planes[2] = {f.clovinv, nullptr};
   pack_clover(g, c->d_inv, prec, inv_planes, 1, c->stream);
@@ -480,19 +488,21 @@ void apply_clover(gbc_ctx* c, int prec, int parity, bool inverse, const Spinor& 
 void ensure_sym(gbc_ctx* c, int prec) {
   ensure_prec(c, prec);
   PrecFields& f = c->pf[pidx(prec)];
-  if (f.clovinv_odd) return;
+  if (f.odd_ready) return;
   if (prec == PREC_DF) {
     ensure_sym(c, PREC_DOUBLE);
     const size_t cb = clover_bytes(PREC_DOUBLE) * c->g.stride;
-    GBC_CUDA(cudaMalloc(&f.clovinv_odd, cb));
+    take(&f.clovinv_odd, cb);
     split_df64((const double*)c->pf[pidx(PREC_DOUBLE)].clovinv_odd, (float2*)f.clovinv_odd, cb / 8, c->stream);
     GBC_CUDA(cudaGetLastError());
+    f.odd_ready = true;
     return;
   }
-  GBC_CUDA(cudaMalloc(&f.clovinv_odd, clover_bytes(prec) * c->g.stride));
+  take(&f.clovinv_odd, clover_bytes(prec) * c->g.stride);
   void* planes[2] = {nullptr, f.clovinv_odd};
   pack_clover(c->g, c->d_inv, prec, planes, 2, c->stream);
   GBC_CUDA(cudaGetLastError());
+  f.odd_ready = true;
 }
 
 // Symmetric even-odd operator (seoprec_clover_linop_w.cc:145-187):
@@ -620,7 +630,7 @@ int gbc_create(gbc_ctx** out, const gbc_geom* geom, const gbc_action* act, const
     GBC_CUDA(cudaMalloc(&c->d_result, sizeof(double) * 3 * c->max_rhs));
     GBC_CUDA(cudaMallocHost(&c->h_result, sizeof(double) * 3 * c->max_rhs));
     GBC_CUDA(cudaMalloc(&c->d_count, sizeof(unsigned) * 4 * c->max_rhs));
-    GBC_CUDA(cudaMemset(c->d_count, 0, sizeof(unsigned) * 4 * c->max_rhs));
+    GBC_CUDA(cudaMemsetAsync(c->d_count, 0, sizeof(unsigned) * 4 * c->max_rhs, c->stream));
     GBC_CUDA(cudaMalloc(&c->d_cg, sizeof(CGScalars) * c->max_rhs));
     GBC_CUDA(cudaMallocHost(&c->h_cg, sizeof(CGScalars) * c->max_rhs));
     GBC_CUDA(cudaMalloc(&c->d_a, sizeof(double) * c->max_rhs));
@@ -660,7 +670,7 @@ void gbc_destroy(gbc_ctx* c) {
 }
 
 static int rebuild_from_clover(gbc_ctx* c) {
-  for (auto& f : c->pf) free_prec(f);
+  for (auto& f : c->pf) f.ready = f.odd_ready = false;  // repacked on next use, in the same buffers
   c->have_gauge = true;
   return GBC_OK;
 }
@@ -681,40 +691,20 @@ int gbc_load_gauge(gbc_ctx* c, const double* links) {
       bool t = a.aniso && (pairs[k][0] == a.t_dir || pairs[k][1] == a.t_dir);
       cc.coef[k] = a.aniso ? (t ? cT : cR) : cR;
     }
-    double* d_logdet = nullptr;
-    int* d_nneg = nullptr;
-    GBC_CUDA(cudaMalloc(&d_logdet, sizeof(double) * V));
-    GBC_CUDA(cudaMalloc(&d_nneg, sizeof(int) * V));
     // A^-1 on both parities: the asymmetric operator needs A_ee^-1, the symmetric one A_oo^-1 too
-    clover_build(c->dims, c->d_links, cc, c->d_clov, c->d_inv, d_logdet, d_nneg, 2, c->stream);
+    const int nb = clover_build(c->dims, c->d_links, cc, c->d_clov, c->d_inv, c->d_partials, c->part_stride, 2, c->stream);
     GBC_CUDA(cudaGetLastError());
-    std::vector<double> ld(V);
-    std::vector<int> nn(V);
-    GBC_CUDA(cudaMemcpyAsync(ld.data(), d_logdet, sizeof(double) * V, cudaMemcpyDeviceToHost, c->stream));
-    GBC_CUDA(cudaMemcpyAsync(nn.data(), d_nneg, sizeof(int) * V, cudaMemcpyDeviceToHost, c->stream));
+    std::vector<double> sums(3 * (size_t)c->part_stride);
+    GBC_CUDA(cudaMemcpyAsync(sums.data(), c->d_partials, sizeof(double) * sums.size(), cudaMemcpyDeviceToHost, c->stream));
     sync(c);
-    cudaFree(d_logdet);
-    cudaFree(d_nneg);
     // log det and negative pivots of A_ee (Chroma's cholesDet(0)); log det of A_oo (cholesDet(1))
-    double s = 0, s_odd = 0;
-    int n = 0;
-    for (long i = 0; i < V; ++i) {
-      long r = i;
-      int par = 0;
-      for (int k = 0; k < 4; ++k) {
-        par += (int)(r % c->dims[k]);
-        r /= c->dims[k];
-      }
-      if (par & 1) {
-        s_odd += ld[i];
-        continue;
-      }
-      s += ld[i];
-      n += nn[i];
-    }
-    c->logdet_even = s;
-    c->logdet_odd = s_odd;
-    c->nneg = n;
+    double s[3] = {0, 0, 0};
+    for (int q = 0; q < 3; ++q)
+      for (int i = 0; i < nb; ++i) s[q] += sums[(size_t)q * c->part_stride + i];
+    c->logdet_even = s[0];
+    c->logdet_odd = s[1];
+    c->nneg = (int)s[2];
+    const int n = c->nneg;
     ++c->gauge_version;
     if (n && c->opts.verbose) fprintf(stderr, "gbclover: WARNING %d negative clover eigenvalues\n", n);
     return rebuild_from_clover(c);
@@ -771,7 +761,7 @@ int gbc_apply(gbc_ctx* c, int op, int isign, int cb, int prec, int nrhs, double*
     const size_t n = (size_t)nrhs * c->V * 24;
     const size_t rs = (size_t)c->V * 24;
     GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], in, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], out, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+    HostResult result(c->stream, copy_stream(c), {{out, c->d_stage[1], n * sizeof(double)}}, HostResult::kLoad);
     const bool dag = isign < 0;
     const PrecFields& f = c->pf[pidx(prec)];
     const int sp = prec == GBC_PREC_DF64 ? GBC_PREC_DOUBLE : prec;  // storage of the spinors
@@ -779,6 +769,7 @@ int gbc_apply(gbc_ctx* c, int op, int isign, int cb, int prec, int nrhs, double*
     Spinor b = sub(workspace(c, 101, sp, nrhs), 0, nrhs);
     Spinor t = sub(workspace(c, 102, sp, nrhs), 0, nrhs);
     Spinor d = sub(workspace(c, 103, sp, nrhs), 0, nrhs);
+    result.ready();  // out's other sites are in place before any export
     switch (op) {
       case GBC_OP_DSLASH:
         import_spinor(c->g, c->d_stage[0], rs, 1 - cb, a, c->stream);
@@ -818,8 +809,9 @@ int gbc_apply(gbc_ctx* c, int op, int isign, int cb, int prec, int nrhs, double*
       }
     }
     GBC_CUDA(cudaGetLastError());
-    GBC_CUDA(cudaMemcpyAsync(out, c->d_stage[1], n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    result.send(0);
     sync(c);
+    result.wait();
     return GBC_OK;
   });
 }
@@ -832,32 +824,21 @@ int gbc_solve(gbc_ctx* c, const gbc_solve_params* p, int nrhs, double* psi, cons
     ensure_stage(c, nrhs);
     const size_t n = (size_t)nrhs * c->V * 24;
     GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], chi, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    // psi is read as the initial guess, and its even sites must survive an odd-parity solve;
-    // only a zero-guess solve of the full system overwrites every site without reading psi
-    if (!(p->zero_guess && p->system == GBC_SYS_FULL))
+    // psi is read as the initial guess, and its even sites must survive an odd-parity solve; only a
+    // zero-guess solve of the full system overwrites every site without reading psi.  A zero-guess
+    // odd-parity solve needs those even sites when it exports its solution, so they are fetched
+    // beside it.
+    if (!p->zero_guess)
       GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], psi, n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     // the solution's copy to the host runs on a second stream as soon as the solution is final,
     // overlapping the FP64 residual check that only reads it
-    if (!c->copy_stream) GBC_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
-    cudaEvent_t exported;
-    GBC_CUDA(cudaEventCreateWithFlags(&exported, cudaEventDisableTiming));
     // (a call refused before the solve starts leaves psi untouched)
-    const std::function<void()> d2h = [&]() {
-      GBC_CUDA(cudaEventRecord(exported, c->stream));
-      GBC_CUDA(cudaStreamWaitEvent(c->copy_stream, exported, 0));
-      GBC_CUDA(cudaMemcpyAsync(psi, c->d_stage[1], n * sizeof(double), cudaMemcpyDeviceToHost, c->copy_stream));
-    };
-    int rc;
-    try {
-      rc = solve_device(c, p, nrhs, c->d_stage[1], c->d_stage[0], res, &d2h);
-    } catch (...) {
-      cudaStreamSynchronize(c->copy_stream);
-      cudaEventDestroy(exported);
-      throw;
-    }
+    HostResult out(c->stream, copy_stream(c), {{psi, c->d_stage[1], n * sizeof(double)}},
+                   p->zero_guess && p->system != GBC_SYS_FULL ? HostResult::kLoad : HostResult::kKeep);
+    const std::function<void()> before = [&]() { out.ready(); }, d2h = [&]() { out.send(0); };
+    const int rc = solve_device(c, p, nrhs, c->d_stage[1], c->d_stage[0], res, &d2h, &before);
     sync(c);
-    GBC_CUDA(cudaStreamSynchronize(c->copy_stream));
-    cudaEventDestroy(exported);
+    out.wait();
     double t1 = now();
     for (int r = 0; r < nrhs; ++r) res[r].seconds = t1 - t0;
     return rc;

@@ -21,12 +21,13 @@ inline int pidx(int prec) {
 }
 
 struct PrecFields {
-  bool ready = false;
+  bool ready = false;  // packed from the present links and clover (the buffers outlive a reload)
   int recon = 18;
   void* gauge[2][4] = {{nullptr}};  // [parity][mu]
   void* clov[2] = {nullptr, nullptr};
   void* clovinv = nullptr;      // A^-1, even parity
   void* clovinv_odd = nullptr;  // A^-1, odd parity (symmetric operator only; packed on first use)
+  bool odd_ready = false;
 };
 
 struct CudaError {
@@ -125,6 +126,7 @@ void free_ctx_memory(gbc_ctx* c);
 void ensure_prec(gbc_ctx* c, int prec);  // pack gauge/clover in this precision
 void ensure_stage(gbc_ctx* c, int nrhs);
 Red red(gbc_ctx* c);
+cudaStream_t copy_stream(gbc_ctx* c);  // the context's second stream, made on first use
 
 // ---- operator blocks on device fields (all of precision prec) ------------------------------
 // out(out_parity) = mode-epilogue of a * D'(in)
@@ -187,7 +189,9 @@ std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const
                                 std::vector<double>& rr, std::vector<int>& status);
 // after_export (optional) runs once the solution is in psi_canon on the context stream and before
 // the final residual check, which only reads it: gbc_solve starts the copy to the host there
+// before_export (optional) runs before the first write to psi_canon of a zero-guess solve
 int solve_device(gbc_ctx* c, const gbc_solve_params* p, int nrhs, double* psi_canon, const double* chi_canon,
-                 gbc_result* res, const std::function<void()>* after_export = nullptr);
+                 gbc_result* res, const std::function<void()>* after_export = nullptr,
+                 const std::function<void()>* before_export = nullptr);
 
 }  // namespace gbc

@@ -1,0 +1,127 @@
+#include "hostmem.h"
+
+#include <sys/mman.h>
+#include <unistd.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <exception>
+
+#include "ctx.h"
+
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23  // Linux 5.14
+#endif
+
+namespace gbc {
+namespace {
+
+// below this a buffer's page faults cost less than a thread
+constexpr size_t kSmall = 2u << 20;
+
+size_t page_size() {
+  const long ps = sysconf(_SC_PAGESIZE);
+  return ps > 0 ? (size_t)ps : 4096;
+}
+
+size_t total_bytes(const PageTouch::Ranges& ranges) {
+  size_t n = 0;
+  for (const auto& r : ranges) n += r.second;
+  return n;
+}
+
+}  // namespace
+
+void PageTouch::populate(Ranges ranges, std::function<void()> then) {
+  join();
+  then_ = std::move(then);
+  if (total_bytes(ranges) < kSmall) return;
+  try {
+    th_[0] = std::thread([this, ranges = std::move(ranges), page = page_size()] {
+      for (const auto& r : ranges) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(r.first) & ~(uintptr_t)(page - 1);
+        const uintptr_t end = reinterpret_cast<uintptr_t>(r.first) + r.second;
+        (void)madvise(reinterpret_cast<void*>(p), end - p, MADV_POPULATE_WRITE);
+      }
+      if (then_) then_();
+      then_ = nullptr;
+    });
+  } catch (const std::exception&) {  // no thread: join() runs `then`
+  }
+}
+
+void PageTouch::overwrite(Ranges ranges) {
+  join();
+  const size_t total = total_bytes(ranges), page = page_size();
+  if (total < kSmall) return;
+  const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
+  // one thread per 8 MB, up to 8 (16 were no faster) and half of the cores
+  const int n = (int)std::min<size_t>(std::min(8, std::max(1, cores / 2)), total / (8u << 20) + 1);
+  try {
+    for (int k = 0; k < n; ++k)
+      th_[k] = std::thread([ranges, page, k, n] {
+        for (const auto& r : ranges) {
+          volatile char* p = static_cast<volatile char*>(r.first);
+          const size_t pages = (r.second + page - 1) / page;
+          for (size_t i = pages * k / n; i < pages * (k + 1) / n; ++i) p[i * page] = 0;
+        }
+      });
+  } catch (const std::exception&) {
+  }
+}
+
+void PageTouch::join() {
+  for (auto& t : th_)
+    if (t.joinable()) t.join();
+  if (then_) then_();
+  then_ = nullptr;
+}
+
+HostResult::HostResult(cudaStream_t work, cudaStream_t copy, std::vector<Item> items, Mode mode)
+    : work_(work), copy_(copy), items_(std::move(items)), load_(mode == kLoad) {
+  GBC_CUDA(cudaGetDevice(&dev_));
+  GBC_CUDA(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
+  PageTouch::Ranges ranges;
+  for (const Item& i : items_) ranges.push_back({i.host, i.bytes});
+  if (mode == kWhole) {
+    touch_.overwrite(std::move(ranges));
+  } else if (mode == kKeep) {
+    touch_.populate(std::move(ranges));
+  } else {
+    // the slots may still be in use by work enqueued before this call
+    GBC_CUDA(cudaEventRecord(ev_, work_));
+    GBC_CUDA(cudaStreamWaitEvent(copy_, ev_, 0));
+    touch_.populate(std::move(ranges), [this] {
+      err_ = cudaSetDevice(dev_);
+      for (const Item& i : items_)
+        if (err_ == cudaSuccess) err_ = cudaMemcpyAsync(i.dev, i.host, i.bytes, cudaMemcpyHostToDevice, copy_);
+    });
+  }
+}
+
+HostResult::~HostResult() {
+  touch_.join();
+  cudaStreamSynchronize(copy_);
+  if (ev_) cudaEventDestroy(ev_);
+}
+
+void HostResult::ready() {
+  if (is_ready_) return;
+  is_ready_ = true;
+  touch_.join();
+  GBC_CUDA(err_);
+  if (!load_) return;
+  GBC_CUDA(cudaEventRecord(ev_, copy_));
+  GBC_CUDA(cudaStreamWaitEvent(work_, ev_, 0));
+}
+
+void HostResult::send(size_t q) {
+  ready();
+  GBC_CUDA(cudaEventRecord(ev_, work_));
+  GBC_CUDA(cudaStreamWaitEvent(copy_, ev_, 0));
+  GBC_CUDA(cudaMemcpyAsync(items_[q].host, items_[q].dev, items_[q].bytes, cudaMemcpyDeviceToHost, copy_));
+}
+
+void HostResult::wait() { GBC_CUDA(cudaStreamSynchronize(copy_)); }
+
+}  // namespace gbc

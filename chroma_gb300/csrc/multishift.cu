@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "hostmem.h"
 
 namespace gbc {
 namespace {
@@ -98,6 +99,10 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
   ensure_stage(c, ns);
   GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], chi_canon, rs * sizeof(double), cudaMemcpyHostToDevice, s));
   import_spinor(g, c->d_stage[0], rs, 1, chid, s);
+  // the solutions go back through d_stage[1], one slot per shift (the even sites of psi_s are kept)
+  std::vector<HostResult::Item> items(ns);
+  for (int q = 0; q < ns; ++q) items[q] = {psi_canon[q], c->d_stage[1] + q * rs, rs * sizeof(double)};
+  HostResult out(s, copy_stream(c), std::move(items), HostResult::kLoad);
   if (mixed) blas_copy(g, chi, chid, s);
   Coefs co(ns), one(1);
 
@@ -222,8 +227,12 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
   cudaEventElapsedTime(&ms, ev0, ev1);
   const long long launches = launch_count() - launches0;
 
-  // true FP64 residual of every shifted system, then the odd sites of each solution to the host
-  // (the even sites of psi_s are kept: the caller's arrays are staged first)
+  // the odd sites of each solution to the host, beside the true FP64 residual of every shifted system
+  out.ready();
+  for (int q = 0; q < ns; ++q) {
+    export_spinor(g, c->d_stage[1] + q * rs, rs, 1, sub(XD, q, 1), s);
+    out.send(q);
+  }
   Spinor t1 = sub(workspace(c, MS_T1, D, 1), 0, 1);
   Spinor t2 = sub(workspace(c, MS_T2, D, 1), 0, 1);
   Spinor ted = sub(workspace(c, MS_TE, D, 1), 0, 1);
@@ -247,11 +256,9 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
     if (o.status == GBC_OK && !(o.rel_resid <= pp->rsd_tolerance_factor * rsd[q])) o.status = GBC_ERR_NOT_CONVERGED;
     o.device_seconds = ms * 1e-3;
     o.launches = (int)launches;
-    GBC_CUDA(cudaMemcpyAsync(c->d_stage[1], psi_canon[q], rs * sizeof(double), cudaMemcpyHostToDevice, s));
-    export_spinor(g, c->d_stage[1], rs, 1, xq, s);
-    GBC_CUDA(cudaMemcpyAsync(psi_canon[q], c->d_stage[1], rs * sizeof(double), cudaMemcpyDeviceToHost, s));
-    sync(c);
   }
+  sync(c);
+  out.wait();
   cudaEventDestroy(ev0);
   cudaEventDestroy(ev1);
   const double t1s = now();

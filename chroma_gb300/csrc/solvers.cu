@@ -741,7 +741,8 @@ std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const
 }
 
 int solve_device(gbc_ctx* c, const gbc_solve_params* pp, int nrhs, double* psi_canon, const double* chi_canon,
-                 gbc_result* res, const std::function<void()>* after_export) {
+                 gbc_result* res, const std::function<void()>* after_export,
+                 const std::function<void()>* before_export) {
   gbc_solve_params p = *pp;
   if (!(p.rsd_target > 0)) p.rsd_target = 1e-10;
   if (p.max_iter <= 0) p.max_iter = 10000;
@@ -1076,6 +1077,7 @@ int solve_device(gbc_ctx* c, const gbc_solve_params* pp, int nrhs, double* psi_c
       rr = fetch(c, 1, n);
     }
   }
+  if (before_export) (*before_export)();
   export_spinor(g, psi_canon, rs, 1, psi, s);
   if (p.system != GBC_SYS_FULL && after_export) (*after_export)();
   if (p.system == GBC_SYS_FULL) {

@@ -22,6 +22,7 @@
 #include <string>
 
 #include "ctx.h"
+#include "hostmem.h"
 
 namespace gbc {
 namespace {
@@ -276,6 +277,11 @@ extern "C" int gbc_stout_smear(const gbc_geom* geom, int n_steps, double rho, co
   double2* buf[2] = {nullptr, nullptr};
   cudaStream_t s = nullptr;
   int rc = GBC_OK;
+  PageTouch touch;
+  try {
+    if (!overlap(links_out, links_in, bytes)) touch.overwrite({{links_out, bytes}});
+  } catch (...) {  // no host memory for the helpers: the copy meets the page faults itself
+  }
   if (cudaMalloc(&buf[0], bytes) != cudaSuccess || cudaMalloc(&buf[1], bytes) != cudaSuccess ||
       cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
     rc = GBC_ERR_CUDA;
@@ -285,6 +291,7 @@ extern "C" int gbc_stout_smear(const gbc_geom* geom, int n_steps, double rho, co
       stout_kernel<<<(unsigned)((g.V + 31) / 32), 128, 0, s>>>(g, buf[i & 1], buf[(i + 1) & 1], rho, dirs);
       count_launch();
     }
+    touch.join();
     cudaMemcpyAsync(links_out, buf[n_steps & 1], bytes, cudaMemcpyDeviceToHost, s);
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = GBC_ERR_CUDA;
   }

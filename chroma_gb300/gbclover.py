@@ -155,10 +155,11 @@ def gauge_synthetic(dims, eps, seed, n_stout=0, rho=0.0, smear_dirs=(1, 1, 1, 1)
 def stout_smear(dims, links, n_steps, rho, smear_dirs=(1, 1, 1, 1)):
     """n_steps stout steps of weight rho on the GPU (FP64); links (V, 4, 3, 3) complex128, no BC."""
     lib = load()
-    u = np.ascontiguousarray(links, dtype=np.complex128).copy()
+    src = np.ascontiguousarray(links, dtype=np.complex128)
+    u = np.empty_like(src)
     g = Geom((C.c_int * 4)(*dims), 1)
     sd = (C.c_int * 4)(*smear_dirs)
-    rc = lib.gbc_stout_smear(C.byref(g), int(n_steps), float(rho), sd, _dp(u.view(np.float64)),
+    rc = lib.gbc_stout_smear(C.byref(g), int(n_steps), float(rho), sd, _dp(src.view(np.float64)),
                              _dp(u.view(np.float64)))
     if rc != GBC_OK:
         raise GBCError(rc, "stout_smear")
@@ -234,7 +235,7 @@ class Context:
     def apply(self, op, x, isign=+1, cb=1, prec=PREC_DOUBLE, out=None):
         x = self._fields(x)
         nrhs = x.shape[0]
-        out = np.zeros_like(x) if out is None else self._fields(out).copy()
+        out = np.zeros(x.shape, x.dtype) if out is None else self._fields(out).copy()
         self._check(self.lib.gbc_apply(self.h, int(op), int(isign), int(cb), int(prec), nrhs,
                                        _dp(out.view(np.float64)), _dp(x.view(np.float64))), "apply")
         return out
@@ -244,7 +245,8 @@ class Context:
               raise_on_error=True, ndefl=0):
         chi = self._fields(chi)
         nrhs = chi.shape[0]
-        psi = np.zeros_like(chi) if psi0 is None else self._fields(psi0).copy()
+        # np.zeros takes fresh pages, which the library makes resident beside the solve (zeros_like fills them here)
+        psi = np.zeros(chi.shape, chi.dtype) if psi0 is None else self._fields(psi0).copy()
         p = SolveParams(int(solver), int(system), float(rsd_target), int(max_iter), float(delta), float(tol_factor),
                         int(sloppy_precision), float(inner_tol), 0, int(nkrylov), int(use_precond),
                         int(psi0 is None), int(ndefl))
@@ -334,7 +336,7 @@ class Context:
 
     def precond_apply(self, x):
         x = self._fields(x)
-        out = np.zeros_like(x)
+        out = np.empty_like(x)  # written entirely, zeros on the even sites
         self._check(self.lib.gbc_precond_apply(self.h, x.shape[0], _dp(out.view(np.float64)),
                                                _dp(x.view(np.float64))), "precond_apply")
         return out
@@ -387,7 +389,7 @@ class Batch:
     def solve(self, chis, rsd_target=1e-10, max_iter=10000, delta=0.1, sloppy_precision=0, inner_tol=0.0):
         n = len(self.contexts)
         chis = [np.ascontiguousarray(x, dtype=np.complex128).reshape(ctx.V, 12) for x, ctx in zip(chis, self.contexts)]
-        psis = [np.zeros_like(x) for x in chis]
+        psis = [np.zeros(x.shape, x.dtype) for x in chis]
         p = SolveParams(SOLVER_MIXED, SYS_MEO, float(rsd_target), int(max_iter), float(delta), 10.0,
                         int(sloppy_precision), float(inner_tol), 0, 16, 0, 1)
         cp = (C.POINTER(C.c_double) * n)(*[_dp(x.view(np.float64)) for x in chis])
