@@ -140,6 +140,31 @@ struct AxpbyF {
   }
 };
 
+// y = a x + b y (as AxpbyF, one precision); acc = |y|^2
+template <typename P>
+struct AxpbyNormF {
+  using Acc = typename P::real;
+  const double2* a;
+  const double2* b;
+  Spinor x, y;
+  __device__ void operator()(int idx, int r, Acc* acc) const {
+    using T = typename P::real;
+    cplx<T> xs[12], ys[12];
+    ld<P>(xs, x, idx, r);
+    ld<P>(ys, y, idx, r);
+    const double2 ca = a[r], cb = b[r];
+    const cplx<T> A{(T)ca.x, (T)ca.y}, B{(T)cb.x, (T)cb.y};
+    T s = 0;
+#pragma unroll
+    for (int k = 0; k < 12; ++k) {
+      ys[k] = A * xs[k] + B * ys[k];
+      s = fmadd(ys[k].re, ys[k].re, fmadd(ys[k].im, ys[k].im, s));
+    }
+    st<P>(y, idx, r, ys);
+    acc[0] += s;
+  }
+};
+
 // x += a p; r -= a q; acc = |r|^2   (x, r in PA;  p, q in PO)
 template <typename PA, typename PO>
 struct CgUpdateF {
@@ -398,6 +423,10 @@ void blas_zero(const Geom& g, const Spinor& y, cudaStream_t s) {
 }
 void blas_axpby(const Geom& g, const double2* a, const Spinor& x, const double2* b, const Spinor& y, cudaStream_t s) {
   GBC_DISPATCH2(y.prec, x.prec, (run<0>(g, y.nrhs, AxpbyF<PA, PB>{a, b, x, y}, nullptr, s)));
+}
+void blas_axpby_norm2(const Geom& g, const double2* a, const Spinor& x, const double2* b, const Spinor& y, const Red& red,
+                      cudaStream_t s) {
+  GBC_DISPATCH1(y.prec, (run<1>(g, y.nrhs, AxpbyNormF<PA>{a, b, x, y}, &red, s)));
 }
 void blas_norm2(const Geom& g, const Spinor& x, const Red& r, cudaStream_t s) {
   GBC_DISPATCH1(x.prec, (run<1>(g, x.nrhs, Norm2F<PA>{x}, &r, s)));

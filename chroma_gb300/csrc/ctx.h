@@ -183,10 +183,11 @@ void bicgstab_xr_update(gbc_ctx* c, int pa, int po, const double* alpha_omega, i
 // FP64 defect correction of the shifted normal systems (M~^dag M~ + sigma_q) psi_q = chi, one per
 // right-hand side q of psi (FP64, holding the initial guesses), the corrections from CG with
 // per-right-hand-side shifts d_shift (device) in the sloppy operator precision; returns the CG
-// iterations per shift, the final FP64 |chi - (M~^dag M~ + sigma_q) psi_q|^2 in rr and a status
+// iterations per shift, the FP64 |chi - (M~^dag M~ + sigma_q) psi_q|^2 in rr (of the returned psi when
+// rr_final) and a status
 std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const double* d_shift,
                                 const Spinor& psi, const std::vector<double>& rsd, int max_iter,
-                                std::vector<double>& rr, std::vector<int>& status);
+                                std::vector<double>& rr, std::vector<int>& status, bool& rr_final);
 // after_export (optional) runs once the solution is in psi_canon on the context stream and before
 // the final residual check, which only reads it: gbc_solve starts the copy to the host there
 // before_export (optional) runs before the first write to psi_canon of a zero-guess solve

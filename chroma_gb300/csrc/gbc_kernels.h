@@ -201,7 +201,7 @@ struct CloverCoeffs {
 };
 // clov[V][72] = packed A (all sites); inv[V][72] = packed A^-1 on the sites of parity inv_parity
 // (2: both parities; zero elsewhere).  sums: per-block partials, in three rows of sums_stride (at
-// least V / 64), of sum log|d_i| of the LDL^dag factors on the even and on the odd sites, and of the
+// least V / 32), of sum log|d_i| of the LDL^dag factors on the even and on the odd sites, and of the
 // number of negative d_i on the even sites; returns the partials per row.
 int clover_build(const int dims[4], const double* canon_links, const CloverCoeffs& cc, double* clov, double* inv,
                  double* sums, int sums_stride, int inv_parity, cudaStream_t s);
@@ -235,6 +235,9 @@ void blas_copy(const Geom& g, const Spinor& y, const Spinor& x, cudaStream_t s);
 void blas_zero(const Geom& g, const Spinor& y, cudaStream_t s);
 void blas_axpby(const Geom& g, const double2* a, const Spinor& x, const double2* b, const Spinor& y,
                 cudaStream_t s);                                                           // y = a x + b y
+// y = a x + b y (x in y's precision), result = |y|^2
+void blas_axpby_norm2(const Geom& g, const double2* a, const Spinor& x, const double2* b, const Spinor& y,
+                      const Red& red, cudaStream_t s);
 void blas_norm2(const Geom& g, const Spinor& x, const Red& r, cudaStream_t s);             // result[0][rhs]
 void blas_cdot(const Geom& g, const Spinor& x, const Spinor& y, const Red& r, cudaStream_t s);  // <x,y> -> result[0..1]
 // CG update: x += a p;  r -= a q;  result = |r|^2      (a per rhs, real)

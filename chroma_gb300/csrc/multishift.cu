@@ -12,6 +12,7 @@
 #include <algorithm>
 #include <cmath>
 #include <string>
+#include <cstring>
 #include <vector>
 
 #include "ctx.h"
@@ -20,7 +21,7 @@
 namespace gbc {
 namespace {
 
-enum { MS_CHI = 700, MS_R, MS_P0, MS_MP, MS_MMP, MS_TE, MS_P, MS_X, MS_T1, MS_T2 };
+enum { MS_CHI = 700, MS_R, MS_MP, MS_MMP, MS_TE, MS_P, MS_X, MS_T1, MS_T2 };
 
 // the first finalized sum of red(c) -> host (synchronises)
 double fetch(gbc_ctx* c) {
@@ -58,6 +59,111 @@ struct Coefs {
   }
 };
 
+// The recursion's scalars on the device, so that iterations run without a host round trip.  Arrays of
+// ns entries behind it: shift, rsd_sq (|chi|^2 target^2), zeta, zeta of the step before, b zeta; conv;
+// and the coefficient arrays of the three updates.
+struct MsScal {
+  double cp, cc, a, b, bp;
+  int done, status, iters, ns;
+  double *shift, *rsd_sq, *z, *zprev, *bs;
+  int* conv;
+  double2* cp_;  // [2][ns + 1]: p_s = zeta_s r + a_s p_s, and p0 = r + a p0 in the last place
+  double2* cr;   // [2]: r = b A p0 + r
+  double2* cx;   // [2][ns]: psi_s -= bs_s p_s
+};
+
+// a = |r|^2 / |r_prev|^2 and the direction coefficients (converged shifts keep p_s: 0, 1)
+__global__ void ms_directions(MsScal* m) {
+  const int n = m->ns, q = threadIdx.x;
+  const bool done = m->done;
+  const double a = done ? 0.0 : m->cc / m->cp, b = m->b;
+  __syncthreads();
+  for (int k = q; k < n; k += blockDim.x) {
+    const bool keep = done || m->conv[k];
+    m->cp_[k] = make_double2(keep ? 0.0 : m->z[k], 0.0);
+    m->cp_[n + 1 + k] = make_double2(keep ? 1.0 : a * m->z[k] * m->bs[k] / (m->zprev[k] * b), 0.0);
+  }
+  if (q == 0) {
+    m->cp_[n] = make_double2(done ? 0.0 : 1.0, 0.0);
+    m->cp_[2 * n + 1] = make_double2(done ? 1.0 : a, 0.0);
+    m->a = a;
+    if (!done) m->cp = m->cc;
+  }
+}
+
+// b = -|r|^2 / <p0, A p0>
+__global__ void ms_step(MsScal* m, const double* d) {
+  if (!m->done) {
+    m->bp = m->b;
+    m->b = -m->cp / d[0];
+  }
+  m->cr[0] = make_double2(m->done ? 0.0 : m->b, 0.0);
+  m->cr[1] = make_double2(1.0, 0.0);
+}
+
+// zeta_next = zeta zeta_prev bp / (b a (zeta_prev - zeta) + zeta_prev bp (1 - sigma b)), the solution
+// coefficients, and convergence of each shift (one block)
+__global__ void ms_solution(MsScal* m, const double* rr) {
+  const int n = m->ns, q = threadIdx.x;
+  const bool done = m->done;
+  const double cc = rr[0], a = m->a, b = m->b, bp = m->bp;
+  int open = 0;
+  for (int k = q; k < n; k += blockDim.x) {
+    const bool skip = done || m->conv[k];
+    if (!skip) {
+      const double z = m->z[k], zp = m->zprev[k];
+      const double zn = z * zp * bp / (b * a * (zp - z) + zp * bp * (1.0 - m->shift[k] * b));
+      m->bs[k] = b * zn / z;
+      m->zprev[k] = z;
+      m->z[k] = zn;
+      m->conv[k] = cc * zn * zn < m->rsd_sq[k];
+    }
+    m->cx[k] = make_double2(skip ? 0.0 : -m->bs[k], 0.0);
+    m->cx[n + k] = make_double2(1.0, 0.0);
+    open |= !m->conv[k];
+  }
+  open = __syncthreads_or(open);
+  if (q == 0 && !done) {
+    m->cc = cc;
+    m->iters += 1;
+    if (!isfinite(cc)) m->status = GBC_ERR_NONFINITE;
+    m->done = !open || !isfinite(cc);
+  }
+}
+
+// the device side of MsScal, one allocation
+struct MsDevice {
+  MsScal h{};
+  MsScal* d = nullptr;
+  void upload(gbc_ctx* c, int ns, const std::vector<double>& shift, const std::vector<double>& rsd_sq,
+              const std::vector<double>& z, const std::vector<double>& zprev, const std::vector<double>& bs) {
+    const size_t nd = 5 * (size_t)ns, n2 = 2 * (ns + 1) + 2 + 2 * (size_t)ns;
+    const size_t head = (sizeof(MsScal) + 15) / 16 * 16, bytes = head + n2 * 16 + nd * 8 + (size_t)ns * 4;
+    GBC_CUDA(cudaMalloc(&d, bytes));
+    char* p = reinterpret_cast<char*>(d) + head;
+    h.cp_ = reinterpret_cast<double2*>(p);
+    h.cr = h.cp_ + 2 * (ns + 1);
+    h.cx = h.cr + 2;
+    h.shift = reinterpret_cast<double*>(h.cx + 2 * (size_t)ns);
+    h.rsd_sq = h.shift + ns;
+    h.z = h.rsd_sq + ns;
+    h.zprev = h.z + ns;
+    h.bs = h.zprev + ns;
+    h.conv = reinterpret_cast<int*>(h.bs + ns);
+    h.ns = ns;
+    std::vector<char> img(bytes, 0);
+    std::memcpy(img.data(), &h, sizeof h);
+    const std::vector<double>* src[5] = {&shift, &rsd_sq, &z, &zprev, &bs};
+    char* base = img.data() + (reinterpret_cast<char*>(h.shift) - reinterpret_cast<char*>(d));
+    for (int k = 0; k < 5; ++k) std::memcpy(base + sizeof(double) * ns * k, src[k]->data(), sizeof(double) * ns);
+    GBC_CUDA(cudaMemcpyAsync(d, img.data(), bytes, cudaMemcpyHostToDevice, c->stream));
+    sync(c);  // img goes out of scope
+  }
+  ~MsDevice() {
+    if (d) cudaFree(d);
+  }
+};
+
 }  // namespace
 
 int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const double* shifts, const double* rsd,
@@ -89,11 +195,11 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
   Spinor chid = sub(workspace(c, MS_CHI, D, 1), 0, 1);
   Spinor chi = mixed ? sub(workspace(c, MS_CHI + o, W, 1), 0, 1) : chid;
   Spinor r = sub(workspace(c, MS_R + o, W, 1), 0, 1);
-  Spinor p0 = sub(workspace(c, MS_P0 + o, W, 1), 0, 1);
   Spinor mp = sub(workspace(c, MS_MP + o, W, 1), 0, 1);
   Spinor mmp = sub(workspace(c, MS_MMP + o, W, 1), 0, 1);
   Spinor te = sub(workspace(c, MS_TE + o, W, 1), 0, 1);
-  Spinor P = sub(workspace(c, MS_P + o, W, ns), 0, ns);
+  Spinor Pall = sub(workspace(c, MS_P + o, W, ns + 1), 0, ns + 1);  // p_s, then p0
+  Spinor P = sub(Pall, 0, ns), p0 = sub(Pall, ns, 1);
   Spinor X = sub(workspace(c, MS_X + o, W, ns), 0, ns);
   const size_t rs = (size_t)c->V * 24;
   ensure_stage(c, ns);
@@ -107,7 +213,6 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
   Coefs co(ns), one(1);
 
   std::vector<double> shift(shifts, shifts + ns), rsd_sq(ns);
-  std::vector<int> conv(ns, 0);
   int k = 0, iters = 0, status = GBC_OK;
   const double chi2 = norm2(c, chi);
   blas_zero(g, X, s);
@@ -143,64 +248,71 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
     co.axpby(c, broadcast(chi, ns), X);
     double cc = norm2(c, r);
     bool done = cc < rsd_sq[smallest];
-    for (k = 1; k <= max_iter && !done; ++k) {
-      if (!std::isfinite(cc)) {
-        status = GBC_ERR_NONFINITE;
-        break;
-      }
-      const double a = cc / cp;
-      // p0 = r + a p0
-      one.h[0] = make_double2(1.0, 0.0);
-      one.h[1] = make_double2(a, 0.0);
-      one.axpby(c, r, p0);
-      // p_s = zeta_s r + as_s p_s  (converged shifts keep p_s: coefficients 0, 1)
-      for (int q = 0; q < ns; ++q) {
-        if (conv[q]) {
-          co.h[q] = make_double2(0.0, 0.0);
-          co.h[ns + q] = make_double2(1.0, 0.0);
-        } else {
-          const double as = a * z[q] * bs[q] / (zprev[q] * b);
-          co.h[q] = make_double2(z[q], 0.0);
-          co.h[ns + q] = make_double2(as, 0.0);
+    if (!done && !std::isfinite(cc)) status = GBC_ERR_NONFINITE;
+    if (!done && status == GBC_OK) {
+      MsDevice ms;
+      ms.h.cp = cp;
+      ms.h.cc = cc;
+      ms.h.b = b;
+      ms.upload(c, ns, shift, rsd_sq, z, zprev, bs);
+      const int nth = std::min(256, (ns + 31) / 32 * 32);
+      auto body = [&]() {
+        ms_directions<<<1, nth, 0, s>>>(ms.d);
+        // p0 = r + a p0 and p_s = zeta_s r + as_s p_s in one pass over r
+        blas_axpby(g, ms.h.cp_, broadcast(r, ns + 1), ms.h.cp_ + ns + 1, Pall, s);
+        apply_meo(c, W, false, p0, mp, te, true);
+        ms_step<<<1, 1, 0, s>>>(ms.d, c->d_result);
+        apply_meo(c, W, true, mp, mmp, te, false);
+        blas_axpby_norm2(g, ms.h.cr, mmp, ms.h.cr + 1, r, red(c), s);  // r += b A p0
+        ms_solution<<<1, nth, 0, s>>>(ms.d, c->d_result);
+        blas_axpby(g, ms.h.cx, P, ms.h.cx + ns, X, s);
+        count_launch(3);
+      };
+      // blocks of iterations between host checks, replayed from a graph after the first (uncaptured,
+      // tuning) iteration; once every shift has converged an iteration changes nothing
+      constexpr int kBlock = 4;
+      cudaGraphExec_t exec = nullptr;
+      struct ExecScope {
+        cudaGraphExec_t& e;
+        ~ExecScope() {
+          if (e) cudaGraphExecDestroy(e);
         }
+      } scope{exec};
+      long long graph_launches = 0;
+      MsScal now_{};
+      while (!now_.done && k < max_iter) {
+        const int steps = k == 0 ? 1 : std::min(kBlock, max_iter - k);
+        if (k > 0 && steps == kBlock && c->use_graphs) {
+          if (!exec) {
+            cudaGraph_t graph;
+            const long long l0 = launch_count();
+            GBC_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+            for (int q = 0; q < kBlock; ++q) body();
+            GBC_CUDA(cudaStreamEndCapture(s, &graph));
+            GBC_CUDA(cudaGraphInstantiate(&exec, graph, 0));
+            cudaGraphDestroy(graph);
+            graph_launches = launch_count() - l0;
+            count_launch(-graph_launches);
+          }
+          GBC_CUDA(cudaGraphLaunch(exec, s));
+          count_launch(graph_launches);
+        } else {
+          for (int q = 0; q < steps; ++q) body();
+        }
+        k += steps;
+        GBC_CUDA(cudaMemcpyAsync(&now_, ms.d, sizeof now_, cudaMemcpyDeviceToHost, s));
+        sync(c);
       }
-      co.axpby(c, broadcast(r, ns), P);
-      cp = cc;
-      apply_meo(c, W, false, p0, mp, te, true);
-      d = fetch(c);
-      apply_meo(c, W, true, mp, mmp, te, false);
-      const double bp = b;
-      b = -cp / d;
-      one.h[0] = make_double2(b, 0.0);
-      one.h[1] = make_double2(1.0, 0.0);
-      one.axpby(c, mmp, r);
-      cc = norm2(c, r);
-      // zeta_next = zeta zeta_prev bp / (b a (zeta_prev - zeta) + zeta_prev bp (1 - sigma b))
-      for (int q = 0; q < ns; ++q) {
-        if (conv[q]) continue;
-        const double zn = z[q] * zprev[q] * bp / (b * a * (zprev[q] - z[q]) + zprev[q] * bp * (1.0 - shift[q] * b));
-        bs[q] = b * zn / z[q];
-        zprev[q] = z[q];
-        z[q] = zn;
-      }
-      // psi_s -= bs_s p_s
-      for (int q = 0; q < ns; ++q) {
-        co.h[q] = make_double2(conv[q] ? 0.0 : -bs[q], 0.0);
-        co.h[ns + q] = make_double2(1.0, 0.0);
-      }
-      co.axpby(c, P, X);
-      done = true;
-      for (int q = 0; q < ns; ++q) {
-        if (!conv[q]) conv[q] = cc * z[q] * z[q] < rsd_sq[q];
-        done = done && conv[q];
-      }
-      iters = k;
+      iters = now_.iters;
+      status = now_.status;
+      done = now_.done && status == GBC_OK;
     }
     if (!done && status == GBC_OK) status = GBC_ERR_NOT_CONVERGED;
   }
   // mixed precision: FP64 copies of the solutions, refined shift by shift (batched)
   std::vector<int> refine_iters(ns, 0), refine_status(ns, GBC_OK);
   std::vector<double> refine_rr;
+  bool rr_final = false;
   Spinor XD = X;
   if (mixed) {
     XD = sub(workspace(c, MS_X, D, ns), 0, ns);
@@ -212,7 +324,7 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
       std::vector<double> rsdv(rsd, rsd + ns);
       try {
         refine_iters = refine_shifted(c, sp, chid, d_shift, XD, rsdv, std::max(1, max_iter - iters), refine_rr,
-                                      refine_status);
+                                      refine_status, rr_final);
       } catch (...) {
         cudaFree(d_shift);
         throw;
@@ -237,14 +349,19 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
   Spinor t2 = sub(workspace(c, MS_T2, D, 1), 0, 1);
   Spinor ted = sub(workspace(c, MS_TE, D, 1), 0, 1);
   for (int q = 0; q < ns; ++q) {
-    Spinor xq = sub(XD, q, 1);
-    apply_meo(c, D, false, xq, t1, ted, false);
-    apply_meo(c, D, true, t1, t2, ted, false);
-    one.h[0] = make_double2(shift[q], 0.0);
-    one.h[1] = make_double2(1.0, 0.0);
-    one.axpby(c, xq, t2);  // t2 = (M~^dag M~ + sigma) psi
-    blas_xmy_norm2(g, chid, t2, red(c), s);
-    const double rr = fetch(c);
+    double rr = 0.0;
+    if (rr_final) {
+      rr = refine_rr[q];  // the refinement ended on this residual of this solution
+    } else {
+      Spinor xq = sub(XD, q, 1);
+      apply_meo(c, D, false, xq, t1, ted, false);
+      apply_meo(c, D, true, t1, t2, ted, false);
+      one.h[0] = make_double2(shift[q], 0.0);
+      one.h[1] = make_double2(1.0, 0.0);
+      one.axpby(c, xq, t2);  // t2 = (M~^dag M~ + sigma) psi
+      blas_xmy_norm2(g, chid, t2, red(c), s);
+      rr = fetch(c);
+    }
     gbc_result& o = res[q];
     o = gbc_result{};
     o.n_count = iters + refine_iters[q];

@@ -672,7 +672,7 @@ CgStats fgmres(gbc_ctx* c, int pa, int po, const Spinor& x, const Spinor& b, dou
 
 std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const double* d_shift,
                                 const Spinor& psi, const std::vector<double>& rsd, int max_iter,
-                                std::vector<double>& rr, std::vector<int>& status) {
+                                std::vector<double>& rr, std::vector<int>& status, bool& rr_final) {
   const int D = PREC_DOUBLE, S = PREC_SINGLE;
   const int n = psi.nrhs;
   const Geom& g = c->g;
@@ -691,6 +691,7 @@ std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const
   status.assign(n, GBC_OK);
   rr.assign(n, 0.0);
   std::vector<double> prev(n, HUGE_VAL);
+  rr_final = false;
   for (int outer = 0; outer < 30; ++outer) {
     // FP64 residual of every shifted system
     apply_sys(c, D, true, psi, r, t1, te);
@@ -719,7 +720,10 @@ std::vector<int> refine_shifted(gbc_ctx* c, int sloppy, const Spinor& chi, const
       worst = std::max(worst, std::sqrt(rr[q] / chi2) / rsd[q]);
       budget = std::min(budget, max_iter - iters[q]);
     }
-    if (!any || budget <= 0) break;
+    if (!any || budget <= 0) {
+      rr_final = true;  // psi has not changed since
+      break;
+    }
     // the correction only needs the part of the reduction still missing (with a factor 2 margin)
     const double itol = std::min(0.1, std::max(1e-6, 0.5 / worst));
     blas_copy(g, rs, r, s);
