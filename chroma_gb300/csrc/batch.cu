@@ -62,6 +62,7 @@ HopArgs make_args(gbc_ctx* c, int prec, int out_parity, int mode, double a, cons
   h.a = a;
   h.twist = twist;
   h.partials = c->d_partials;
+  h.active = &c->d_cg[0].active;  // a converged lattice's blocks return at once
   h.part_stride = c->part_stride;
   (void)mode;
   return h;

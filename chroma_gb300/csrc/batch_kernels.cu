@@ -59,7 +59,7 @@ template <typename PA, typename PO>
 __global__ void __launch_bounds__(kSites) update_kernel(const LatCg* lat, const int2* work) {
   const int2 w = work[blockIdx.x];
   const LatCg& l = lat[w.x];
-  batch_update_block<PA, PO>(l, w.y, l.cg->a);
+  if (l.cg->active) batch_update_block<PA, PO>(l, w.y, l.cg->a);  // a converged lattice is frozen
 }
 
 // p = r + b p   (r in PA, p in PO)
@@ -67,7 +67,7 @@ template <typename PA, typename PO>
 __global__ void __launch_bounds__(kSites) xpay_kernel(const LatCg* lat, const int2* work) {
   const int2 w = work[blockIdx.x];
   const LatCg& l = lat[w.x];
-  batch_xpay_block<PA, PO>(l, w.y, l.cg->b);
+  if (l.cg->active) batch_xpay_block<PA, PO>(l, w.y, l.cg->b);
 }
 
 }  // namespace
