@@ -235,9 +235,11 @@ constexpr int kTmemCols = 32;  // tensor-memory columns allocated per block (>= 
 // channel and right-hand side and writes 16 bytes per shared-memory store.  A 12 -> 12 layer at
 // 16^3 x 32: 1772 -> 492 us for 12 right-hand sides, 217 -> 60 us for one (kernel time, cold L2).
 // IN_ODD: only the self term of odd sites and the hops of even sites are non-zero; the others'
-// columns of G are zeroed once, and odd sites need only the K steps that cover the self term.
+// columns of G are zeroed, and odd sites need only the K steps that cover the self term.
+// A block walks its tiles: weights, tensor memory and barrier are set up once, and warps 3..8 gather
+// the next tile while warps 0..2 still store this one.
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int batch, int per, int flags,
+__global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int total, int batch, int per, int flags,
                                                       const float2* __restrict__ links, const float4* __restrict__ hin,
                                                       float4* __restrict__ hout, const uint4* __restrict__ Wc) {
   constexpr int KP = kpad(CIN), NP = npad(COUT), NU = nump(COUT);
@@ -251,11 +253,6 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, d = tid >> 5, s = tid & 31;
-  int tile = blockIdx.x, par = 1;
-  if (!(flags & OUT_ODD)) {
-    par = tile >= tiles ? 1 : 0;
-    tile -= par * tiles;
-  }
   const int b0 = blockIdx.y * per, b1 = min(batch, b0 + per);
   for (int p = tid; p < NP * KP / 8; p += CT) reinterpret_cast<uint4*>(W)[p] = __ldg(Wc + p);
   if (d == 0) {
@@ -268,75 +265,86 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" ::"r"(smem_u32(&mbar)));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  const int i = tile * SITES + s;
-  const bool valid = i < g.Vh;
-  const int ic = valid ? i : g.Vh - 1;  // lanes past the end gather the last site, store nothing
-  const int j = par * g.Vh + ic;
-  const bool mine = !(flags & IN_ODD) || ((d == 0) == (par == 1));
-  const int n = neighbour(g, par, ic, d);
-  float2 m[9];
-  if (mine && d > 0) load_transport(m, links, V, j, n, d);
   constexpr int CH = CIN / 4;  // 16-byte chunks of a direction
-  if (!mine) {
-#pragma unroll
-    for (int c = 0; c < CH; ++c)
-#pragma unroll
-      for (int a = 0; a < 3; ++a)
-        *reinterpret_cast<uint4*>(G + core_row<KP>(a * 32 + s, d * CH + c)) = make_uint4(0, 0, 0, 0);
-  }
   if (KP > 18 * CIN && d == 0) {
 #pragma unroll
     for (int a = 0; a < 3; ++a)
       *reinterpret_cast<uint4*>(G + core_row<KP>(a * 32 + s, DIRS * CH)) = make_uint4(0, 0, 0, 0);
   }
-  const int ksteps = (flags & IN_ODD) && par == 1 ? (2 * CIN + 15) / 16 : KP / 16;
   const uint64_t adesc = umma_desc(smem_u32(G), 128, KP * 16);
   const uint64_t bdesc = umma_desc(smem_u32(W), 128, KP * 16);
   constexpr uint32_t idesc = umma_idesc_bf16(MROWS, NU);
-  bool ok = true;
-  for (int b = b0; b < b1; ++b) {
-    if (mine) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
-    // the tensor cores read G and W through the async proxy
-    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-    // every thread leaves together once a wait for the previous right-hand side has given up
-    if (!__syncthreads_and(ok)) break;
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = tmem_base;
-    if (tid == 0) {
-      for (int ks = 0; ks < ksteps; ++ks) {
-        // K steps of 16 elements: two core matrices along K, 256 bytes
-        const uint64_t da = adesc + (uint64_t)((ks * 256) >> 4), db = bdesc + (uint64_t)((ks * 256) >> 4);
-        const uint32_t acc = ks > 0 ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-            "l"(da), "l"(db), "r"(idesc), "r"(acc));
-      }
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
-                       smem_u32(&mbar))
-                   : "memory");
+  bool ok = true, dead = false;
+  uint32_t phase = 0;  // of the block's next MMA on the mbarrier
+  for (int t = blockIdx.x; t < total && !dead; t += gridDim.x) {
+    int tile = t, par = 1;
+    if (!(flags & OUT_ODD)) {
+      par = tile >= tiles ? 1 : 0;
+      tile -= par * tiles;
     }
-    // every thread waits: the MMA has read G (the next gather may overwrite it) and written its
-    // accumulators
-    const uint32_t phase = (uint32_t)((b - b0) & 1);
-    ok = mbar_wait(smem_u32(&mbar), phase);
-    if (!ok) {
-      if (tid == 0) atomicAdd(&g_tc_wait_errors, 1);
-      // give the MMAs in flight one more bounded wait before their tensor memory is freed
-      (void)mbar_wait(smem_u32(&mbar), phase);
-      continue;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    if (d < 3) {  // warp = colour, lane = site
-      float v[NU];
-      tmem_load_row<NU>(tmem + ((uint32_t)(d * 32) << 16), v);
-      if (valid) {
-        float4* out = hout + (size_t)b * V * planes(COUT) + j;
+    const int i = tile * SITES + s;
+    const bool valid = i < g.Vh;
+    const int ic = valid ? i : g.Vh - 1;  // lanes past the end gather the last site, store nothing
+    const int j = par * g.Vh + ic;
+    const bool mine = !(flags & IN_ODD) || ((d == 0) == (par == 1));
+    const int n = neighbour(g, par, ic, d);
+    float2 m[9];
+    if (mine && d > 0) load_transport(m, links, V, j, n, d);
+    if (!mine) {
 #pragma unroll
-        for (int q = 0; q < COUT / 2; ++q)
-          out[(size_t)(d * (COUT / 2) + q) * V] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+      for (int c = 0; c < CH; ++c)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+          *reinterpret_cast<uint4*>(G + core_row<KP>(a * 32 + s, d * CH + c)) = make_uint4(0, 0, 0, 0);
+    }
+    const int ksteps = (flags & IN_ODD) && par == 1 ? (2 * CIN + 15) / 16 : KP / 16;
+    for (int b = b0; b < b1; ++b) {
+      if (mine) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
+      // the tensor cores read G and W through the async proxy
+      asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+      // every thread leaves together once a wait for the previous MMA has given up
+      if (!__syncthreads_and(ok)) {
+        dead = true;
+        break;
       }
-      asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      const uint32_t tmem = tmem_base;
+      if (tid == 0) {
+        for (int ks = 0; ks < ksteps; ++ks) {
+          // K steps of 16 elements: two core matrices along K, 256 bytes
+          const uint64_t da = adesc + (uint64_t)((ks * 256) >> 4), db = bdesc + (uint64_t)((ks * 256) >> 4);
+          const uint32_t acc = ks > 0 ? 1u : 0u;
+          asm volatile(
+              "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
+              "l"(da), "l"(db), "r"(idesc), "r"(acc));
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
+                         smem_u32(&mbar))
+                     : "memory");
+      }
+      // every thread waits: the MMA has read G (the next gather may overwrite it) and written its
+      // accumulators
+      ok = mbar_wait(smem_u32(&mbar), phase);
+      if (!ok) {
+        if (tid == 0) atomicAdd(&g_tc_wait_errors, 1);
+        // give the MMAs in flight one more bounded wait before their tensor memory is freed
+        (void)mbar_wait(smem_u32(&mbar), phase);
+      }
+      phase ^= 1;
+      if (!ok) continue;
+      asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+      if (d < 3) {  // warp = colour, lane = site
+        float v[NU];
+        tmem_load_row<NU>(tmem + ((uint32_t)(d * 32) << 16), v);
+        if (valid) {
+          float4* out = hout + (size_t)b * V * planes(COUT) + j;
+#pragma unroll
+          for (int q = 0; q < COUT / 2; ++q)
+            out[(size_t)(d * (COUT / 2) + q) * V] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+      }
     }
   }
   __syncthreads();
@@ -619,8 +627,9 @@ void launch_layer(const Geom& g, int V, int batch, int flags, const float2* link
   const size_t smem = (size_t)128 * kpad(CIN) * 2;
   GBC_CUDA(cudaFuncSetAttribute(layer_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const Split w = split_of(g, batch, flags);
-  layer_kernel<CIN, COUT><<<dim3(w.blocks, w.parts), CT, smem, s>>>(g, V, w.tiles, batch, w.per, flags, links, in, out,
-                                                                    reinterpret_cast<const uint4*>(W));
+  // three resident blocks per SM
+  layer_kernel<CIN, COUT><<<dim3(std::min(w.blocks, 3 * 152), w.parts), CT, smem, s>>>(
+      g, V, w.tiles, w.blocks, batch, w.per, flags, links, in, out, reinterpret_cast<const uint4*>(W));
   count_launch();
 }
 
