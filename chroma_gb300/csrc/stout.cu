@@ -23,47 +23,10 @@
 
 #include "ctx.h"
 #include "hostmem.h"
+#include "su3.cuh"
 
 namespace gbc {
 namespace {
-
-struct M {
-  double2 a[9];
-};
-
-// r += x y
-__device__ __forceinline__ void mac(double2& r, double2 x, double2 y) {
-  r.x = fma(x.x, y.x, r.x);
-  r.x = fma(-x.y, y.y, r.x);
-  r.y = fma(x.x, y.y, r.y);
-  r.y = fma(x.y, y.x, r.y);
-}
-__device__ __forceinline__ double2 cj(double2 x) { return make_double2(x.x, -x.y); }
-
-// r += X Y with X = x or x^dag, Y = y or y^dag
-template <bool XD, bool YD>
-__device__ __forceinline__ void mmac(M& r, const M& x, const M& y) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-        mac(r.a[3 * i + j], XD ? cj(x.a[3 * k + i]) : x.a[3 * i + k], YD ? cj(y.a[3 * j + k]) : y.a[3 * k + j]);
-}
-__device__ __forceinline__ M mzero() {
-  M r;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) r.a[k] = make_double2(0.0, 0.0);
-  return r;
-}
-__device__ __forceinline__ M ld(const double2* u, long site, int mu) {
-  M r;
-  const double2* p = u + (site * 4 + mu) * 9;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) r.a[k] = __ldg(p + k);
-  return r;
-}
 
 // Hermitian 3x3: diagonal d, upper off-diagonals o[0] = 01, o[1] = 02, o[2] = 12
 struct Herm {
@@ -202,31 +165,14 @@ __global__ void __launch_bounds__(128) stout_kernel(Lat g, const double2* __rest
   if (!on[mu]) {
     out = ld(cur, s, mu);
   } else {
-    // the site's neighbours: s + up[k] and s + dn[k]
-    long up[4], dn[4], r = s, stride = 1;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int x = (int)(r % g.L[k]);
-      r /= g.L[k];
-      up[k] = x + 1 == g.L[k] ? -stride * (g.L[k] - 1) : stride;
-      dn[k] = x == 0 ? stride * (g.L[k] - 1) : -stride;
-      stride *= g.L[k];
-    }
-    long up_mu = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (k == mu) up_mu = up[k];
+    int x[4];
+    const Steps n = steps(g.L, s, x);
+    const long up_mu = pick(n.up, mu);
     M C = mzero();
 #pragma unroll 1
     for (int nu = 0; nu < 4; ++nu) {
       if (nu == mu || !on[nu]) continue;
-      long un = 0, dnn = 0;
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (k == nu) {
-          un = up[k];
-          dnn = dn[k];
-        }
+      const long un = pick(n.up, nu), dnn = pick(n.dn, nu);
       // a step in nu leaves the mu coordinate alone: x - nu + mu is s + dnn + up_mu
       M t = mzero();
       mmac<false, false>(t, ld(cur, s, nu), ld(cur, s + un, mu));
