@@ -25,6 +25,7 @@ __device__ double block_sum(const double* part, int n) {
 }
 
 __global__ void __launch_bounds__(256) alpha_kernel(const LatCg* lat) {
+  pdl_begin();
   const LatCg& l = lat[blockIdx.x];
   const double d = block_sum(l.hop_part, l.nblk);
   if (threadIdx.x == 0) {
@@ -36,6 +37,7 @@ __global__ void __launch_bounds__(256) alpha_kernel(const LatCg* lat) {
 }
 
 __global__ void __launch_bounds__(256) beta_kernel(const LatCg* lat) {
+  pdl_begin();
   const LatCg& l = lat[blockIdx.x];
   const double cp = block_sum(l.upd_part, l.nblk);
   if (threadIdx.x == 0) {
@@ -57,6 +59,7 @@ __global__ void __launch_bounds__(256) beta_kernel(const LatCg* lat) {
 // e += a p;  r -= a q;  partial |r|^2 per block   (e, r in PA; p, q in PO)
 template <typename PA, typename PO>
 __global__ void __launch_bounds__(kSites) update_kernel(const LatCg* lat, const int2* work) {
+  pdl_begin();
   const int2 w = work[blockIdx.x];
   const LatCg& l = lat[w.x];
   if (l.cg->active) batch_update_block<PA, PO>(l, w.y, l.cg->a);  // a converged lattice is frozen
@@ -65,6 +68,7 @@ __global__ void __launch_bounds__(kSites) update_kernel(const LatCg* lat, const 
 // p = r + b p   (r in PA, p in PO)
 template <typename PA, typename PO>
 __global__ void __launch_bounds__(kSites) xpay_kernel(const LatCg* lat, const int2* work) {
+  pdl_begin();
   const int2 w = work[blockIdx.x];
   const LatCg& l = lat[w.x];
   if (l.cg->active) batch_xpay_block<PA, PO>(l, w.y, l.cg->b);
@@ -75,17 +79,17 @@ __global__ void __launch_bounds__(kSites) xpay_kernel(const LatCg* lat, const in
 // the precision pairs a batch uses: (FP64, FP64) for an FP64 sloppy operator, else FP32
 // accumulators with an FP32 or FP16 stencil
 #define GBC_PAIR_LAUNCH(KERNEL)                                                  \
-  if (pa == PREC_DOUBLE) KERNEL<PrecD, PrecD><<<nwork, kSites, 0, s>>>(lat, work); \
-  else if (po == PREC_SINGLE) KERNEL<PrecS, PrecS><<<nwork, kSites, 0, s>>>(lat, work); \
-  else KERNEL<PrecS, PrecH><<<nwork, kSites, 0, s>>>(lat, work);                   \
+  if (pa == PREC_DOUBLE) launch_pdl(KERNEL<PrecD, PrecD>, nwork, kSites, s, lat, work); \
+  else if (po == PREC_SINGLE) launch_pdl(KERNEL<PrecS, PrecS>, nwork, kSites, s, lat, work); \
+  else launch_pdl(KERNEL<PrecS, PrecH>, nwork, kSites, s, lat, work);                   \
   count_launch();
 
 void batch_cg_alpha(const LatCg* lat, int n, cudaStream_t s) {
-  alpha_kernel<<<n, 256, 0, s>>>(lat);
+  launch_pdl(alpha_kernel, n, 256, s, lat);
   count_launch();
 }
 void batch_cg_beta(const LatCg* lat, int n, cudaStream_t s) {
-  beta_kernel<<<n, 256, 0, s>>>(lat);
+  launch_pdl(beta_kernel, n, 256, s, lat);
   count_launch();
 }
 void batch_cg_update(int pa, int po, const LatCg* lat, const int2* work, int nwork, cudaStream_t s) {

@@ -17,9 +17,8 @@
 // host reports the solve as failed; no wait is unbounded.  A cooperative launch guarantees that
 // every block is resident, so the barrier is only a guard against the unexpected.
 //
-// This file is compiled with GBC_COHERENT_LOADS: spinor fields, which other blocks of the same
-// launch wrote before a barrier, are read with plain loads instead of ld.global.nc (links and
-// clover, which nothing writes, keep the read-only path).
+// Spinor fields, which other blocks of the same launch wrote before a barrier, are read with plain
+// loads (ldw); links and clover, which nothing writes, keep the read-only path.
 #pragma once
 #include <algorithm>
 

@@ -1,5 +1,4 @@
 // Persistent batched CGNE with an fp16 stencil (FP32 accumulators), both link reconstructions.
-#define GBC_COHERENT_LOADS 1
 #include "batch_persistent.cuh"
 
 namespace gbc {

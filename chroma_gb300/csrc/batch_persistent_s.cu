@@ -1,6 +1,5 @@
 // Persistent batched CGNE with an FP32 stencil, both link reconstructions, and the dispatch over
 // the precision pairs (FP64 sloppy batches have no persistent variant: per-launch path).
-#define GBC_COHERENT_LOADS 1
 #include "batch_persistent.cuh"
 #include "ctx.h"
 

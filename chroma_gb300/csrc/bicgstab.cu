@@ -50,19 +50,19 @@ __device__ __forceinline__ void ld4(cplx<typename P::real> (&x)[4], const Spinor
     const double2* p = reinterpret_cast<const double2*>(base);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const double2 v = ldg(p + (size_t)(4 * c + q) * f.stride + idx);
+      const double2 v = ldw(p + (size_t)(4 * c + q) * f.stride + idx);
       x[q] = {v.x, v.y};
     }
   } else if constexpr (std::is_same<P, PrecS>::value) {
     const float4* p = reinterpret_cast<const float4*>(base);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const float4 v = ldg(p + (size_t)(2 * c + h) * f.stride + idx);
+      const float4 v = ldw(p + (size_t)(2 * c + h) * f.stride + idx);
       x[2 * h] = {v.x, v.y};
       x[2 * h + 1] = {v.z, v.w};
     }
   } else {
-    const uint4 v = ldg(reinterpret_cast<const uint4*>(base) + (size_t)c * f.stride + idx);
+    const uint4 v = ldw(reinterpret_cast<const uint4*>(base) + (size_t)c * f.stride + idx);
     const float2 a = h2f(v.x), b = h2f(v.y), d = h2f(v.z), e = h2f(v.w);
     x[0] = {a.x * n, a.y * n};
     x[1] = {b.x * n, b.y * n};
@@ -88,7 +88,7 @@ __device__ __forceinline__ void st4(const Spinor& f, int idx, int r, int c, cons
 }
 template <typename P>
 __device__ __forceinline__ float site_norm(const Spinor& f, int idx, int r) {
-  if constexpr (std::is_same<P, PrecH>::value) return ldg(f.norm + (size_t)r * f.norm_rhs_stride + idx);
+  if constexpr (std::is_same<P, PrecH>::value) return ldw(f.norm + (size_t)r * f.norm_rhs_stride + idx);
   return 1.0f;
 }
 
@@ -99,6 +99,7 @@ __device__ __forceinline__ float site_norm(const Spinor& f, int idx, int r) {
 template <int NRED, class F>
 __global__ void __launch_bounds__(BT, F::kMinb) bi_site_kernel(int Vh, F f, const BiScal* sc, double* partials,
                                                                int part_stride, int nrhs, Finish fin) {
+  pdl_begin();
   using A = typename AccOf<F>::type;  // thread and warp sums in the compute precision
   const int r = blockIdx.y;
   if (!sc[r].active) return;  // uniform over the block
@@ -243,8 +244,7 @@ void run(gbc_ctx* c, int nrhs, const BiScal* sc, const F& f, const Red& rd) {
   const Geom& g = c->g;
   dim3 grid(blas_blocks(g), nrhs);
   const bool inside = NRED > 0 && rd.count && finish_in_kernel((long)grid.x * nrhs);
-  bi_site_kernel<NRED, F><<<grid, BT, 0, c->stream>>>(g.Vh, f, sc, rd.partials, rd.part_stride, nrhs,
-                                                      inside ? rd.finish() : Finish{});
+  launch_pdl(bi_site_kernel<NRED, F>, grid, BT, c->stream, g.Vh, f, sc, rd.partials, rd.part_stride, nrhs, inside ? rd.finish() : Finish{});
   count_launch();
   if (NRED > 0 && !inside) reduce_finalize(rd, NRED, nrhs, grid.x, c->stream);
 }

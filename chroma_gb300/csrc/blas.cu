@@ -19,6 +19,7 @@ constexpr int BLAS_THREADS = 256;
 template <int NRED, class F>
 __global__ void __launch_bounds__(BLAS_THREADS) site_kernel(int Vh, F f, double* partials, int part_stride, int nrhs,
                                                             Finish fin) {
+  pdl_begin();
   using A = typename AccOf<F>::type;
   const int r = blockIdx.y;
   A acc[NRED > 0 ? NRED : 1];
@@ -345,6 +346,7 @@ struct XsubNormF {
 
 __global__ void finalize_kernel(const double* partials, int part_stride, int nblocks, double* result) {
   // one block per (quantity, rhs); fixed-order tree => bitwise repeatable
+  pdl_begin();
   const int qr = blockIdx.x;
   __shared__ double sh[256];
   double s = 0.0;
@@ -362,6 +364,7 @@ __global__ void finalize_kernel(const double* partials, int part_stride, int nbl
 template <int NQ>
 __global__ void __launch_bounds__(256) finish_kernel(Finish f, const double* partials, int part_stride, int nrhs,
                                                      int nblocks) {
+  pdl_begin();
   sum_partials<NQ, 256>(f, partials, part_stride, nrhs, blockIdx.x, nblocks);
 }
 
@@ -369,9 +372,8 @@ template <int NRED, class F>
 void run(const Geom& g, int nrhs, const F& f, const Red* red, cudaStream_t s) {
   dim3 grid(blas_blocks(g), nrhs);
   const bool inside = NRED > 0 && red->count && finish_in_kernel((long)grid.x * nrhs);
-  site_kernel<NRED, F><<<grid, BLAS_THREADS, 0, s>>>(g.Vh, f, red ? red->partials : nullptr,
-                                                     red ? red->part_stride : 0, nrhs,
-                                                     inside ? red->finish() : Finish{});
+  launch_pdl(site_kernel<NRED, F>, grid, BLAS_THREADS, s, g.Vh, f, red ? red->partials : nullptr,
+             red ? red->part_stride : 0, nrhs, inside ? red->finish() : Finish{});
   count_launch();
   if (NRED > 0 && !inside) reduce_finalize(*red, NRED, nrhs, grid.x, s);
 }
@@ -386,10 +388,11 @@ int blas_blocks(const Geom& g) {
 }
 
 void reduce_finalize(const Red& red, int nred, int nrhs, int nblocks, cudaStream_t s) {
-  if (red.kind == FIN_SUM) finalize_kernel<<<nred * nrhs, 256, 0, s>>>(red.partials, red.part_stride, nblocks, red.result);
-  else if (nred == 1) finish_kernel<1><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
-  else if (nred == 2) finish_kernel<2><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
-  else finish_kernel<3><<<nrhs, 256, 0, s>>>(red.finish(), red.partials, red.part_stride, nrhs, nblocks);
+  if (red.kind == FIN_SUM)
+    launch_pdl(finalize_kernel, nred * nrhs, 256, s, red.partials, red.part_stride, nblocks, red.result);
+  else if (nred == 1) launch_pdl(finish_kernel<1>, nrhs, 256, s, red.finish(), red.partials, red.part_stride, nrhs, nblocks);
+  else if (nred == 2) launch_pdl(finish_kernel<2>, nrhs, 256, s, red.finish(), red.partials, red.part_stride, nrhs, nblocks);
+  else launch_pdl(finish_kernel<3>, nrhs, 256, s, red.finish(), red.partials, red.part_stride, nrhs, nblocks);
   count_launch();
 }
 

@@ -509,6 +509,7 @@ void ensure_sym(gbc_ctx* c, int prec) {
     take(&f.clovinv_odd, cb);
     split_df64((const double*)c->pf[pidx(PREC_DOUBLE)].clovinv_odd, (float2*)f.clovinv_odd, cb / 8, c->stream);
     GBC_CUDA(cudaGetLastError());
+    sync(c);
     f.odd_ready = true;
     return;
   }
@@ -516,6 +517,7 @@ void ensure_sym(gbc_ctx* c, int prec) {
   void* planes[2] = {nullptr, f.clovinv_odd};
   pack_clover(c->g, c->d_inv, prec, planes, 2, c->stream);
   GBC_CUDA(cudaGetLastError());
+  sync(c);  // stencil kernels read it on the read-only path, possibly placed early (launch.cuh)
   f.odd_ready = true;
 }
 

@@ -735,6 +735,7 @@ __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, in
 
 template <typename P, int RECON, int MODE, bool DAG, int REDUCE, int TX, int NRB, int MINB>
 __global__ void __launch_bounds__(TX * NRB, MINB) hop_kernel(const HopArgs a) {
+  pdl_begin();
   const int ng = (a.nrhs + NRB - 1) / NRB;
   const int sblock = blockIdx.x / ng;
   hop_body<P, RECON, MODE, DAG, REDUCE, TX, NRB>(a, sblock, blockIdx.x - sblock * ng);
@@ -744,6 +745,7 @@ __global__ void __launch_bounds__(TX * NRB, MINB) hop_kernel(const HopArgs a) {
 // partials): block b works on lattice work[b].x, site block work[b].y.
 template <typename P, int RECON, int MODE, bool DAG, int REDUCE>
 __global__ void __launch_bounds__(128) hop_kernel_multi(const HopArgs* __restrict__ args, const int2* __restrict__ work) {
+  pdl_begin();
   const int2 w = work[blockIdx.x];
   hop_body<P, RECON, MODE, DAG, REDUCE, 128, 1>(args[w.x], w.y, 0);
 }
@@ -887,8 +889,8 @@ __device__ __forceinline__ void load_project_pair(C2 (&h)[2][3], const void* bas
   uint32_t wa[12], wb[12];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const uint4 va = ldg(p + (size_t)k * stride + ja);
-    const uint4 vb = ldg(p + (size_t)k * stride + jb);
+    const uint4 va = ldw(p + (size_t)k * stride + ja);
+    const uint4 vb = ldw(p + (size_t)k * stride + jb);
     wa[4 * k] = va.x; wa[4 * k + 1] = va.y; wa[4 * k + 2] = va.z; wa[4 * k + 3] = va.w;
     wb[4 * k] = vb.x; wb[4 * k + 1] = vb.y; wb[4 * k + 2] = vb.z; wb[4 * k + 3] = vb.w;
   }
@@ -1014,7 +1016,7 @@ __device__ __forceinline__ void hop_dir_pair(C2 (&acc)[12], const HopArgs& a, co
     nb.x[MU] = cb.x[MU] == last ? 0 : cb.x[MU] + 1;
     const int ja = cb_index(g, na), jb = cb_index(g, nb);
     load_project_pair<MU, SF>(h, in, ja, jb, g.stride);
-    const float2 n = make_float2(ldg(in_norm + ja), ldg(in_norm + jb));
+    const float2 n = make_float2(ldw(in_norm + ja), ldw(in_norm + jb));
     const float ts = (float)g.t_sign;
     const float2 sign = make_float2(ca.x[3] == g.L[3] - 1 ? ts : 1.f, cb.x[3] == g.L[3] - 1 ? ts : 1.f);
     load_link_pair<RECON, MU == 3>(u, a.gauge_fwd[MU], ia, ib, g.stride, sign);
@@ -1026,7 +1028,7 @@ __device__ __forceinline__ void hop_dir_pair(C2 (&acc)[12], const HopArgs& a, co
     nb.x[MU] = cb.x[MU] == 0 ? last : cb.x[MU] - 1;
     const int ja = cb_index(g, na), jb = cb_index(g, nb);
     load_project_pair<MU, SB>(h, in, ja, jb, g.stride);
-    const float2 n = make_float2(ldg(in_norm + ja), ldg(in_norm + jb));
+    const float2 n = make_float2(ldw(in_norm + ja), ldw(in_norm + jb));
     const float ts = (float)g.t_sign;
     const float2 sign = make_float2(na.x[3] == g.L[3] - 1 ? ts : 1.f, nb.x[3] == g.L[3] - 1 ? ts : 1.f);
     load_link_pair<RECON, MU == 3>(u, a.gauge_bwd[MU], ja, jb, g.stride, sign);
@@ -1037,6 +1039,7 @@ __device__ __forceinline__ void hop_dir_pair(C2 (&acc)[12], const HopArgs& a, co
 // Grid: Vh/2 / TX site blocks x nrhs, right-hand sides fastest (as hop_kernel with NRB = 1).
 template <int RECON, int MODE, bool DAG, int REDUCE, int TX, int MINB>
 __global__ void __launch_bounds__(TX, MINB) hop_kernel_pair(const HopArgs a) {
+  pdl_begin();
   const int sblock = blockIdx.x / a.nrhs;
   const int rhs = blockIdx.x - sblock * a.nrhs;
   const Geom& g = a.g;

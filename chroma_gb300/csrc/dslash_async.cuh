@@ -141,6 +141,7 @@ __device__ __forceinline__ void ring_step(float2 (&acc)[12], HopRing<RECON, TX>&
 template <int RECON, int MODE, bool DAG, int REDUCE, int TX, int MINB>
 __global__ void __launch_bounds__(TX, MINB) hop_kernel_async(const HopArgs a) {
   __shared__ HopRing<RECON, TX> R;
+  pdl_begin();
   const int sblock = blockIdx.x / a.nrhs;
   const int rhs = blockIdx.x - sblock * a.nrhs;
   const Geom& g = a.g;

@@ -13,7 +13,7 @@ static int hop_shape(const HopArgs& a, HopShape sh, cudaStream_t s) {
   const int nbx = (a.g.Vh + sh.tx - 1) / sh.tx;
   auto go = [&](auto kern, int tx, int nrb) {
     const int ng = (a.nrhs + nrb - 1) / nrb;
-    kern<<<(unsigned)(nbx * ng), tx * nrb, 0, s>>>(a);
+    launch_pdl(kern, (unsigned)(nbx * ng), tx * nrb, s, a);
     return nbx;
   };
 #define GBC_SHAPE(TX, NRB, MINB)                                 \
@@ -42,7 +42,7 @@ static int hop_shape(const HopArgs& a, HopShape sh, cudaStream_t s) {
 #define GBC_RPAIR(TS, NRB, MINB)                                                          \
   if (sh.tx == TS && sh.nrb == NRB && sh.minb == MINB) {                                  \
     const int ng = (a.nrhs + NRB - 1) / NRB;                                              \
-    hop_kernel_rp<RECON, MODE, DAG, REDUCE, TS, NRB, MINB><<<(unsigned)(nbx * ng), TS * NRB / 2, 0, s>>>(a); \
+    launch_pdl(hop_kernel_rp<RECON, MODE, DAG, REDUCE, TS, NRB, MINB>, (unsigned)(nbx * ng), TS * NRB / 2, s, a); \
     return nbx;                                                                           \
   }
       GBC_RPAIR(32, 12, 2)
@@ -58,7 +58,7 @@ static int hop_shape(const HopArgs& a, HopShape sh, cudaStream_t s) {
       if (a.g.L[3] & 1) return -1;
       auto go2 = [&](auto kern, int tx) {
         const int nbp = (a.g.Vh / 2 + tx - 1) / tx;
-        kern<<<(unsigned)(nbp * a.nrhs), tx, 0, s>>>(a);
+        launch_pdl(kern, (unsigned)(nbp * a.nrhs), tx, s, a);
         return nbp;
       };
 #define GBC_PAIR(TX, MINB) \
@@ -133,12 +133,12 @@ static int hop_recon(int recon, int mode, int reduce, const HopArgs& a, HopShape
 template <typename P, int RECON, bool DAG>
 static int hop_multi_mode(int mode, int reduce, const HopArgs* args, const int2* work, int nwork, cudaStream_t s) {
   switch (mode) {
-    case HOP_PLAIN: hop_kernel_multi<P, RECON, HOP_PLAIN, DAG, RED_NONE><<<nwork, 128, 0, s>>>(args, work); return nwork;
-    case HOP_CLOV: hop_kernel_multi<P, RECON, HOP_CLOV, DAG, RED_NONE><<<nwork, 128, 0, s>>>(args, work); return nwork;
+    case HOP_PLAIN: launch_pdl(hop_kernel_multi<P, RECON, HOP_PLAIN, DAG, RED_NONE>, nwork, 128, s, args, work); return nwork;
+    case HOP_CLOV: launch_pdl(hop_kernel_multi<P, RECON, HOP_CLOV, DAG, RED_NONE>, nwork, 128, s, args, work); return nwork;
     case HOP_XPAY:
       if (reduce == RED_DOT_SELF || reduce == RED_DOT_AUX) return -1;
-      if (reduce) hop_kernel_multi<P, RECON, HOP_XPAY, DAG, RED_NORM><<<nwork, 128, 0, s>>>(args, work);
-      else hop_kernel_multi<P, RECON, HOP_XPAY, DAG, RED_NONE><<<nwork, 128, 0, s>>>(args, work);
+      if (reduce) launch_pdl(hop_kernel_multi<P, RECON, HOP_XPAY, DAG, RED_NORM>, nwork, 128, s, args, work);
+      else launch_pdl(hop_kernel_multi<P, RECON, HOP_XPAY, DAG, RED_NONE>, nwork, 128, s, args, work);
       return nwork;
   }
   return -1;

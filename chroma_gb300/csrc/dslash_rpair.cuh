@@ -64,8 +64,8 @@ __device__ __forceinline__ void load_project_rp(C2 (&h)[2][3], const void* b0, c
   uint32_t w0[12], w1[12];
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const uint4 v0 = ldg(p0 + (size_t)k * stride + j);
-    const uint4 v1 = ldg(p1 + (size_t)k * stride + j);
+    const uint4 v0 = ldw(p0 + (size_t)k * stride + j);
+    const uint4 v1 = ldw(p1 + (size_t)k * stride + j);
     w0[4 * k] = v0.x; w0[4 * k + 1] = v0.y; w0[4 * k + 2] = v0.z; w0[4 * k + 3] = v0.w;
     w1[4 * k] = v1.x; w1[4 * k + 1] = v1.y; w1[4 * k + 2] = v1.z; w1[4 * k + 3] = v1.w;
   }
@@ -125,13 +125,13 @@ __device__ __forceinline__ void hop_dir_rp(C2 (&acc)[12], const float4 (*lsm)[9]
   {
     const int j = nsm[2 * MU][s];
     load_project_rp<MU, SF>(h, in0, in1, j, stride);
-    const float2 n = make_float2(ldg(nm0 + j), ldg(nm1 + j));
+    const float2 n = make_float2(ldw(nm0 + j), ldw(nm1 + j));
     mult_rebuild_rp<MU, SF, TS>(acc, lsm[2 * MU], s, h, n);
   }
   {
     const int j = nsm[2 * MU + 1][s];
     load_project_rp<MU, SB>(h, in0, in1, j, stride);
-    const float2 n = make_float2(ldg(nm0 + j), ldg(nm1 + j));
+    const float2 n = make_float2(ldw(nm0 + j), ldw(nm1 + j));
     mult_rebuild_rp<MU, SB, TS>(acc, lsm[2 * MU + 1], s, h, n);
   }
 }
@@ -181,6 +181,7 @@ template <int RECON, int MODE, bool DAG, int REDUCE, int TS, int NRB, int MINB>
 __global__ void __launch_bounds__(TS * NRB / 2, MINB) hop_kernel_rp(const HopArgs a) {
   static_assert(TS % 16 == 0 && NRB % 4 == 0, "TS sites in half-warps, pair groups in lane pairs");
   constexpr int SW = TS / 16;
+  pdl_begin();
   const int ng = (a.nrhs + NRB - 1) / NRB;
   const int sblock = blockIdx.x / ng;
   const int group = blockIdx.x - sblock * ng;

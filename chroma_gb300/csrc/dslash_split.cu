@@ -8,6 +8,7 @@ namespace {
 // Grid: one dimension, right-hand sides fastest (blocks that share links run together).
 template <int MODE, bool DAG, int REDUCE, int S>
 __global__ void __launch_bounds__(8 * S) hop_kernel_split(const HopArgs a) {
+  pdl_begin();
   const int sblock = blockIdx.x / a.nrhs, rhs = blockIdx.x - sblock * a.nrhs;
   double sum[3] = {0.0, 0.0, 0.0};
   if (!a.active || a.active[(size_t)rhs * a.active_stride])
@@ -21,9 +22,9 @@ template <int MODE, bool DAG, int REDUCE>
 int launch(const HopArgs& a, int sites, cudaStream_t s) {
   const int nb = (a.g.Vh + sites - 1) / sites;
   const unsigned grid = (unsigned)nb * a.nrhs;
-  if (sites == 8) hop_kernel_split<MODE, DAG, REDUCE, 8><<<grid, 64, 0, s>>>(a);
-  else if (sites == 16) hop_kernel_split<MODE, DAG, REDUCE, 16><<<grid, 128, 0, s>>>(a);
-  else hop_kernel_split<MODE, DAG, REDUCE, 32><<<grid, 256, 0, s>>>(a);
+  if (sites == 8) launch_pdl(hop_kernel_split<MODE, DAG, REDUCE, 8>, grid, 64, s, a);
+  else if (sites == 16) launch_pdl(hop_kernel_split<MODE, DAG, REDUCE, 16>, grid, 128, s, a);
+  else launch_pdl(hop_kernel_split<MODE, DAG, REDUCE, 32>, grid, 256, s, a);
   return nb;
 }
 

@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "gbc_kernels.h"
+#include "launch.cuh"
 
 namespace gbc {
 
@@ -233,17 +234,12 @@ __device__ __forceinline__ uint32_t f2h(float a, float b) {
 // Loads of data that no kernel writes while it runs (links, clover, tables): the read-only path.
 template <typename T>
 __device__ __forceinline__ T ldg(const T* p) { return __ldg(p); }
-// Loads of spinor fields and their norms.  Translation units whose kernels read fields that other
-// blocks of the same launch wrote (the persistent batch kernel, between its grid barriers) define
-// GBC_COHERENT_LOADS: plain loads, which the barrier's gpu-scope fences order after those writes;
-// the read-only path (ld.global.nc) requires data that no one writes while the kernel runs.
-#ifdef GBC_COHERENT_LOADS
+// Loads of spinor fields and their norms: plain loads.  A kernel may be resident while its predecessor
+// still writes them (launch.cuh), and the persistent batch kernel reads between its grid barriers what
+// other blocks of the launch wrote; the read-only path (ld.global.nc) requires data that no one writes
+// while the kernel runs, and its loads may be moved above a wait.
 template <typename T>
 __device__ __forceinline__ T ldw(const T* p) { return *p; }
-#else
-template <typename T>
-__device__ __forceinline__ T ldw(const T* p) { return __ldg(p); }
-#endif
 
 // ---- spinor load/store -------------------------------------------------------------------------
 template <typename P>

@@ -13,6 +13,7 @@ constexpr int KT = 256;
 template <typename PV, typename PW>
 __global__ void __launch_bounds__(KT) multi_cdot_kernel(int Vh, VecList vl, Spinor w, double* partials, int part_stride,
                                                        int nrhs) {
+  pdl_begin();
   const int r = blockIdx.y;
   const int i = blockIdx.z;
   const Spinor& v = vl.v[i];
@@ -60,6 +61,7 @@ __global__ void __launch_bounds__(KT) multi_cdot_kernel(int Vh, VecList vl, Spin
 template <typename PV, typename PW>
 __global__ void __launch_bounds__(KT) multi_caxpy_kernel(int Vh, VecList vl, int k, const double2* coef, Spinor w,
                                                         double sign) {
+  pdl_begin();
   const int r = blockIdx.y;
   const int nrhs = gridDim.y;
   using T = typename PW::real;
@@ -85,6 +87,7 @@ __global__ void __launch_bounds__(KT) multi_caxpy_kernel(int Vh, VecList vl, int
 // y = a x (y is not read)
 template <typename PY, typename PX>
 __global__ void __launch_bounds__(KT) cax_kernel(int Vh, const double2* a, Spinor x, Spinor y) {
+  pdl_begin();
   const int r = blockIdx.y;
   using T = typename PY::real;
   const double2 ca = a[r];
@@ -117,7 +120,7 @@ __global__ void __launch_bounds__(KT) cax_kernel(int Vh, const double2* a, Spino
 void multi_cdot(const Geom& g, const VecList& vl, int k, const Spinor& w, const Red& red, cudaStream_t s) {
   dim3 grid(blas_blocks(g), w.nrhs, k);
   GBC_K_DISPATCH2(vl.v[0].prec, w.prec,
-                  (multi_cdot_kernel<PA, PB><<<grid, KT, 0, s>>>(g.Vh, vl, w, red.partials, red.part_stride, w.nrhs)));
+                  (launch_pdl(multi_cdot_kernel<PA, PB>, grid, KT, s, g.Vh, vl, w, red.partials, red.part_stride, w.nrhs)));
   count_launch();
   reduce_finalize(red, 2 * k, w.nrhs, grid.x, s);
 }
@@ -126,13 +129,13 @@ void multi_caxpy(const Geom& g, const VecList& vl, int k, const double2* coef, c
                  cudaStream_t s) {
   dim3 grid(blas_blocks(g), w.nrhs);
   GBC_K_DISPATCH2(vl.v[0].prec, w.prec,
-                  (multi_caxpy_kernel<PA, PB><<<grid, KT, 0, s>>>(g.Vh, vl, k, coef, w, sign)));
+                  (launch_pdl(multi_caxpy_kernel<PA, PB>, grid, KT, s, g.Vh, vl, k, coef, w, sign)));
   count_launch();
 }
 
 void blas_cax(const Geom& g, const double2* a, const Spinor& x, const Spinor& y, cudaStream_t s) {
   dim3 grid(blas_blocks(g), y.nrhs);
-  GBC_K_DISPATCH2(y.prec, x.prec, (cax_kernel<PA, PB><<<grid, KT, 0, s>>>(g.Vh, a, x, y)));
+  GBC_K_DISPATCH2(y.prec, x.prec, (launch_pdl(cax_kernel<PA, PB>, grid, KT, s, g.Vh, a, x, y)));
   count_launch();
 }
 

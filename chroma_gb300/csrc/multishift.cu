@@ -17,6 +17,7 @@
 
 #include "ctx.h"
 #include "hostmem.h"
+#include "launch.cuh"
 
 namespace gbc {
 namespace {
@@ -74,6 +75,7 @@ struct MsScal {
 
 // a = |r|^2 / |r_prev|^2 and the direction coefficients (converged shifts keep p_s: 0, 1)
 __global__ void ms_directions(MsScal* m) {
+  pdl_begin();
   const int n = m->ns, q = threadIdx.x;
   const bool done = m->done;
   const double a = done ? 0.0 : m->cc / m->cp, b = m->b;
@@ -93,6 +95,7 @@ __global__ void ms_directions(MsScal* m) {
 
 // b = -|r|^2 / <p0, A p0>
 __global__ void ms_step(MsScal* m, const double* d) {
+  pdl_begin();
   if (!m->done) {
     m->bp = m->b;
     m->b = -m->cp / d[0];
@@ -104,6 +107,7 @@ __global__ void ms_step(MsScal* m, const double* d) {
 // zeta_next = zeta zeta_prev bp / (b a (zeta_prev - zeta) + zeta_prev bp (1 - sigma b)), the solution
 // coefficients, and convergence of each shift (one block)
 __global__ void ms_solution(MsScal* m, const double* rr) {
+  pdl_begin();
   const int n = m->ns, q = threadIdx.x;
   const bool done = m->done;
   const double cc = rr[0], a = m->a, b = m->b, bp = m->bp;
@@ -257,14 +261,14 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
       ms.upload(c, ns, shift, rsd_sq, z, zprev, bs);
       const int nth = std::min(256, (ns + 31) / 32 * 32);
       auto body = [&]() {
-        ms_directions<<<1, nth, 0, s>>>(ms.d);
+        launch_pdl(ms_directions, 1, nth, s, ms.d);
         // p0 = r + a p0 and p_s = zeta_s r + as_s p_s in one pass over r
         blas_axpby(g, ms.h.cp_, broadcast(r, ns + 1), ms.h.cp_ + ns + 1, Pall, s);
         apply_meo(c, W, false, p0, mp, te, true);
-        ms_step<<<1, 1, 0, s>>>(ms.d, c->d_result);
+        launch_pdl(ms_step, 1, 1, s, ms.d, c->d_result);
         apply_meo(c, W, true, mp, mmp, te, false);
         blas_axpby_norm2(g, ms.h.cr, mmp, ms.h.cr + 1, r, red(c), s);  // r += b A p0
-        ms_solution<<<1, nth, 0, s>>>(ms.d, c->d_result);
+        launch_pdl(ms_solution, 1, nth, s, ms.d, c->d_result);
         blas_axpby(g, ms.h.cx, P, ms.h.cx + ns, X, s);
         count_launch(3);
       };

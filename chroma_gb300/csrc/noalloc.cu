@@ -66,6 +66,7 @@ struct CanonField {
 // even sites: scratch[cb] = A_ee^-1 D'_eo psi_o
 template <bool DAG, int S>
 __global__ void __launch_bounds__(8 * S) noalloc_even(const CanonField<0> f) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the odd kernel may be placed
   double sum[3];
   split_site<CanonField<0>, HOP_CLOV, DAG, RED_NONE, S>(f, 1.0, 0.0, blockIdx.x, sum);
 }
@@ -73,6 +74,7 @@ __global__ void __launch_bounds__(8 * S) noalloc_even(const CanonField<0> f) {
 // odd sites: out = A_oo psi_o - 1/4 D'_oe scratch  (+ isign i mu gamma_5 psi_o)
 template <bool DAG, int S>
 __global__ void __launch_bounds__(8 * S) noalloc_odd(const CanonField<1> f, double twist) {
+  pdl_begin();
   double sum[3];
   split_site<CanonField<1>, HOP_XPAY, DAG, RED_NONE, S>(f, -0.25, twist, blockIdx.x, sum);
 }
@@ -81,7 +83,9 @@ template <bool DAG, int S>
 void noalloc_launch(const CanonField<0>& fe, const CanonField<1>& fo, double twist, cudaStream_t s) {
   const unsigned blocks = (unsigned)((fe.g.Vh + S - 1) / S);
   noalloc_even<DAG, S><<<blocks, 8 * S, 0, s>>>(fe);
-  noalloc_odd<DAG, S><<<blocks, 8 * S, 0, s>>>(fo, twist);
+  // up to two blocks per SM the odd kernel is placed beside the even one (8^4: 24.6 -> 22.5 us); larger
+  // grids would lose their even spread over the SMs
+  launch_pdl_if(blocks <= 2 * 152, noalloc_odd<DAG, S>, blocks, 8 * S, s, fo, twist);
 }
 template <bool DAG>
 void noalloc_launch(const CanonField<0>& fe, const CanonField<1>& fo, double twist, cudaStream_t s) {
