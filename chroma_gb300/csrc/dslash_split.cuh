@@ -120,7 +120,7 @@ __device__ __forceinline__ void split_site(const A& f, double coef, double twist
 #pragma unroll
     for (int t = 0; t < 3; ++t) {
       const int r = 3 * q + t, im = r & 1, spin = r / 6, col = (r >> 1) - 3 * spin;
-      double v = 0.0;
+      double v;
 #pragma unroll
       for (int hp = 0; hp < 8; ++hp) {
         const int mu = hp >> 1;
@@ -134,10 +134,11 @@ __device__ __forceinline__ void split_site(const A& f, double coef, double twist
           minus = minus != neg;
         }
         const double2 w = uh[hp][3 * (hi ? 1 : 0) + col][s];
-        v += flip_if(minus, (im != 0) != cross ? w.y : w.x);
+        const double x = flip_if(minus, (im != 0) != cross ? w.y : w.x);
+        v = hp == 0 ? x : v + x;
       }
       acc[t] = v;
-      if (MODE == HOP_CLOV) xs[r][s] = coef * v;
+      if (MODE == HOP_CLOV) xs[r][s] = coef == 1.0 ? v : coef * v;
     }
   }
   double2 x[6];
