@@ -816,7 +816,7 @@ void Cnn::forward(gbc_ctx* c, int batch) {
 
 // A layer whose wait for its tensor-core results gave up (it then frees its tensor memory and
 // returns) counts in g_tc_wait_errors: read and reset it, and fail the call that ran the layers.
-static void check_tc_waits(cudaStream_t s) {
+void cnn_check_waits(cudaStream_t s) {
   int n = 0;
   GBC_CUDA(cudaMemcpyFromSymbolAsync(&n, g_tc_wait_errors, sizeof(int), 0, cudaMemcpyDeviceToHost, s));
   GBC_CUDA(cudaStreamSynchronize(s));
@@ -849,7 +849,7 @@ double Cnn::loss_and_grad(gbc_ctx* c, int batch) {
   }
   double loss = 0;
   GBC_CUDA(cudaMemcpyAsync(&loss, dl, sizeof(double), cudaMemcpyDeviceToHost, s));
-  check_tc_waits(s);
+  cnn_check_waits(s);
   return loss;
 }
 
@@ -974,7 +974,6 @@ void cnn_apply_spinor(gbc_ctx* c, Cnn& net, const Spinor& in, const Spinor& out)
   else if (out.prec == PREC_SINGLE) extract_kernel<PrecS><<<grid, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
   else extract_kernel<PrecH><<<grid, 128, 0, c->stream>>>(c->g, V, net.act[net.nlayers], out);
   count_launch();
-  check_tc_waits(c->stream);
 }
 
 void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float4* act, double* norm2) {

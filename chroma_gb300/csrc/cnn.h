@@ -52,7 +52,10 @@ struct Cnn {
   void release();
 };
 
+// (the caller runs cnn_check_waits before it relies on the result)
 void cnn_apply_spinor(gbc_ctx* c, Cnn& net, const Spinor& in, const Spinor& out);
+// waits for the stream and throws if a layer gave up waiting for the tensor cores since the last check
+void cnn_check_waits(cudaStream_t s);
 // norm2 (may be null): |f_b|^2 of each field over the odd sites, summed in FP64
 void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float4* act, double* norm2 = nullptr);
 void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float4* act, double* canon_dev);

@@ -158,6 +158,8 @@ int noalloc_reserve();
 void precond_free(gbc_ctx* c);
 // out ~= M~^-1 in (odd checkerboard fields, same precision, nrhs right-hand sides)
 void precond_apply(gbc_ctx* c, const Spinor& in, const Spinor& out);
+// throws if a network layer gave up a wait since the last check (synchronises)
+void precond_check(gbc_ctx* c);
 // layers of the loaded network and the channels of layer l (its output side when out)
 int precond_layers(gbc_ctx* c);
 int precond_channels(gbc_ctx* c, int l, bool out);

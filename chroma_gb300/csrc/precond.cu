@@ -31,6 +31,10 @@ void precond_apply(gbc_ctx* c, const Spinor& in, const Spinor& out) {
   cnn_apply_spinor(c, *n, in, out);
 }
 
+void precond_check(gbc_ctx* c) {
+  if (c->precond) cnn_check_waits(c->stream);
+}
+
 int precond_layers(gbc_ctx* c) { return c->precond ? net_of(c)->nlayers : 0; }
 int precond_channels(gbc_ctx* c, int l, bool out) { return out ? net_of(c)->cout(l) : net_of(c)->cin(l); }
 
@@ -135,6 +139,7 @@ int gbc_precond_apply(gbc_ctx* c, int nrhs, double* out, const double* in) {
     cnn_embed_canon(c, n, nrhs, c->d_stage[0], n.act[0]);
     n.forward(c, nrhs);
     cnn_extract_canon(c, n, nrhs, n.act[n.nlayers], c->d_stage[1]);
+    cnn_check_waits(c->stream);
     res.send(0);
     res.wait();
     sync(c);

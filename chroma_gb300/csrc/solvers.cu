@@ -658,6 +658,7 @@ CgStats fgmres(gbc_ctx* c, int pa, int po, const Spinor& x, const Spinor& b, dou
       eta_prev[i] = e;
     }
     if (jmax > 0) {
+      if (prec) precond_check(c);  // once per cycle, before its directions enter the solution
       put_coef(eta, jmax);
       multi_caxpy(g, Z, jmax, c->d_kcoef, x, 1.0, s);
     }

@@ -94,6 +94,7 @@ extern "C" int gbc_time_operator(gbc_ctx* c, int op, int prec, int nrhs, int ite
       total += ms * 1e-3;
     }
     GBC_CUDA(cudaGetLastError());
+    if (op == GBC_TIME_PRECOND) precond_check(c);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (junk) cudaFree(junk);
