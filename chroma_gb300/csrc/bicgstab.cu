@@ -147,30 +147,6 @@ struct SUpdF {
   }
 };
 
-// (t, s) and |t|^2
-template <typename PO>
-struct TsTtF {
-  static constexpr int kMinb = std::is_same<PO, PrecD>::value ? 2 : 4;
-  using Acc = typename PO::real;
-  Spinor t, s;
-  __device__ void operator()(int idx, int k, Acc* acc) const {
-    using T = typename PO::real;
-    cplx<T> ts[12], ss[12];
-    ldv<PO>(ts, t, idx, k);
-    ldv<PO>(ss, s, idx, k);
-    T re = 0, im = 0, tt = 0;
-#pragma unroll
-    for (int q = 0; q < 12; ++q) {
-      re = fmadd(ts[q].re, ss[q].re, fmadd(ts[q].im, ss[q].im, re));
-      im = fmadd(ts[q].re, ss[q].im, fmadd(-ts[q].im, ss[q].re, im));
-      tt = fmadd(ts[q].re, ts[q].re, fmadd(ts[q].im, ts[q].im, tt));
-    }
-    acc[0] += re;
-    acc[1] += im;
-    acc[2] += tt;
-  }
-};
-
 // x += alpha p + omega (r - alpha v);  r -= alpha v + omega t;  |r|^2 and (r0, r).  Six vectors
 // in and two out per site: processed four colour-spin components at a time (a whole site of all
 // eight would hold ~150 registers and leave one block per SM for a bandwidth-bound loop).
@@ -255,7 +231,7 @@ void iteration(gbc_ctx* c, int po, BiScal* sc, int n, const Spinor& x, const Spi
   const Red rd = red(c);
   // alpha from (r0, v)
   const Red alpha = rd.then(FIN_BI_ALPHA, sc);
-  if (!c->sym && r0.prec == PREC_SINGLE) {
+  if (r0.prec == PREC_SINGLE) {
     // (r0, v) summed in the epilogue of the stencil launch that writes v = M~ p (r0 at its sites)
     c->hop_aux = r0;
     apply_meo(c, po, false, p, v, te, RED_DOT_AUX, &alpha);
@@ -267,13 +243,8 @@ void iteration(gbc_ctx* c, int po, BiScal* sc, int n, const Spinor& x, const Spi
   run<0>(c, n, sc, SUpdF<PA, PO>{sc, r, v, s}, rd);
   // omega from (t, s) and (t, t)
   const Red omega = rd.then(FIN_BI_OMEGA, sc);
-  if (c->sym) {
-    apply_meo(c, po, false, s, t, te, RED_NONE);
-    run<3>(c, n, sc, TsTtF<PO>{t, s}, omega);
-  } else {
-    // both summed in the epilogue of the stencil launch that writes t (s is its self)
-    apply_meo(c, po, false, s, t, te, RED_DOT_SELF, &omega);
-  }
+  // both summed in the epilogue of the stencil launch that writes t (s is its self)
+  apply_meo(c, po, false, s, t, te, RED_DOT_SELF, &omega);
   run<3>(c, n, sc, XRUpdF<PA, PO>{sc, x, r, p, v, t, r0}, rd.then(FIN_BI_BETA, sc));
   run<0>(c, n, sc, PUpdF<PA, PO>{sc, r, p, v}, rd);
 }

@@ -292,7 +292,8 @@ int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce,
   // GBC_SHAPE=<index into kHopShapes> pins one shape (profiling); ignored when out of range
   if (const char* fs = getenv("GBC_SHAPE")) {
     const int si = atoi(fs);
-    if (si >= 0 && si < kNumHopShapes && hop_shape_valid(kHopShapes[si], prec, h.nrhs, h.g.L[3])) {
+    if (si >= 0 && si < kNumHopShapes && hop_shape_valid(kHopShapes[si], prec, h.nrhs, h.g.L[3]) &&
+        hop_shape_for_mode(kHopShapes[si], mode)) {
       c->tuned[key] = si;
       return si;
     }
@@ -333,7 +334,8 @@ int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce,
       for (int si = 0; si < kNumHopShapes; ++si) {
         const HopShape& sh = kHopShapes[si];
         if (sh.tx == t[0] && sh.nrb == t[1] && sh.minb == t[2] && sh.pair == t[3] &&
-            hop_shape_valid(sh, prec, h.nrhs, h.g.L[3]) && hop_blocks(sh, h.g.Vh) <= h.part_stride) {
+            hop_shape_valid(sh, prec, h.nrhs, h.g.L[3]) && hop_shape_for_mode(sh, mode) &&
+            hop_blocks(sh, h.g.Vh) <= h.part_stride) {
           char line[160];
           snprintf(line, sizeof line, "prec=%d mode=%d dag=%d reduce=%d nrhs=%d -> tx=%d nrb=%d minb=%d pair=%d (%s)\n",
                    prec, mode, dag ? 1 : 0, reduce, h.nrhs, sh.tx, sh.nrb, sh.minb, sh.pair, origin);
@@ -359,7 +361,9 @@ int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce,
     std::vector<int> cand;
     for (int si = 0; si < kNumHopShapes; ++si) {
       const HopShape sh = kHopShapes[si];
-      if (!hop_shape_valid(sh, prec, h.nrhs, h.g.L[3]) || hop_blocks(sh, h.g.Vh) > h.part_stride) continue;
+      if (!hop_shape_valid(sh, prec, h.nrhs, h.g.L[3]) || !hop_shape_for_mode(sh, mode) ||
+          hop_blocks(sh, h.g.Vh) > h.part_stride)
+        continue;
       if (launch(si) < 0) continue;
       if (cudaPeekAtLastError() != cudaSuccess) {
         cudaGetLastError();  // e.g. too many resources for this shape: not a candidate
@@ -522,30 +526,31 @@ void ensure_sym(gbc_ctx* c, int prec) {
 }
 
 // Symmetric even-odd operator (seoprec_clover_linop_w.cc:145-187):
-//   PLUS   out = in - 1/4 A_oo^-1 D_oe A_ee^-1 D_eo in     (t_e, then the clover-inverse epilogue)
-//   MINUS  out = in - 1/4 D_oe^dag A_ee^-1 D_eo^dag A_oo^-1 in
-// The last step leaves 1/4 (...) in out and blas_xmy_norm2 turns it into in - out with |out|^2;
-// with a twisted-mass term, in - out + isign i mu gamma_5 in (seoprec_clover_linop_w.cc:174-184:
-// the clover term and its inverses carry no twist, the term is added to M_s itself).
+//   PLUS   out = in - 1/4 A_oo^-1 D_oe A_ee^-1 D_eo in     (two stencil launches, as M~; the reductions of
+//          the solvers are summed in the second one's epilogue)
+//   MINUS  out = in - 1/4 D_oe^dag A_ee^-1 D_eo^dag A_oo^-1 in: the last step leaves 1/4 (...) in out and
+//          blas_xmy_norm2 turns it into in - out with |out|^2
+// With a twisted-mass term, + isign i mu gamma_5 in (seoprec_clover_linop_w.cc:174-184: the clover
+// term and its inverses carry no twist, the term is added to M_s itself).
 void apply_seo(gbc_ctx* c, int prec, bool dag, const Spinor& in, const Spinor& out, const Spinor& tmp_e,
                int reduce, const Red* rd) {
   ensure_sym(c, prec);
   const PrecFields& f = c->pf[pidx(prec)];
   if (!dag) {
     hop(c, prec, 0, HOP_CLOV, false, 1.0, in, tmp_e, nullptr, f.clovinv, false);
-    hop(c, prec, 1, HOP_CLOV, false, 0.25, tmp_e, out, nullptr, f.clovinv_odd, false);
-  } else {
-    Spinor to = sub(workspace(c, 900 + pidx(prec), prec, in.nrhs), 0, in.nrhs);
-    blas_clover(c->g, f.clovinv_odd, to, in, c->stream);
-    hop(c, prec, 0, HOP_CLOV, true, 1.0, to, tmp_e, nullptr, f.clovinv, false);
-    hop(c, prec, 1, HOP_PLAIN, true, 0.25, tmp_e, out, nullptr, nullptr, false);
+    hop(c, prec, 1, HOP_SYM, false, 0.25, tmp_e, out, &in, f.clovinv_odd, reduce, c->act.twisted ? c->act.twisted_m : 0.0,
+        rd);
+    return;
   }
+  Spinor to = sub(workspace(c, 900 + pidx(prec), prec, in.nrhs), 0, in.nrhs);
+  blas_clover(c->g, f.clovinv_odd, to, in, c->stream);
+  hop(c, prec, 0, HOP_CLOV, true, 1.0, to, tmp_e, nullptr, f.clovinv, false);
+  hop(c, prec, 1, HOP_PLAIN, true, 0.25, tmp_e, out, nullptr, nullptr, false);
   const Red sums = rd ? *rd : red(c);
   if (c->act.twisted && c->act.twisted_m != 0.0)
-    blas_xmy_twist_norm2(c->g, in, out, dag ? -c->act.twisted_m : c->act.twisted_m, sums, c->stream);
+    blas_xmy_twist_norm2(c->g, in, out, -c->act.twisted_m, sums, c->stream);
   else
     blas_xmy_norm2(c->g, in, out, sums, c->stream);
-  (void)reduce;
 }
 
 }  // namespace gbc

@@ -11,6 +11,8 @@
 //   HOP_PLAIN  out = a * D' psi
 //   HOP_CLOV   out = T (a * D' psi)                  T = packed clover blocks at the output parity
 //                                                    (A_ee^-1 for  A_ee^-1 D_eo psi_o)
+//   HOP_SYM    out = self - T (a * D' psi)  [+ isign * i * mu * gamma_5 self]
+//                                                    (psi_o - 1/4 A_oo^-1 D_oe t_e, seoprec_clover_linop_w.cc:145-187)
 //   HOP_XPAY   out = T self + a * D' psi  [+ isign * i * mu * gamma_5 self]
 //                                                    (A_oo psi_o - 1/4 D_oe t_e, eoprec_clover_linop_w.cc:142-187)
 //   REDUCE adds per-block partial sums of |out|^2 for each right-hand side.
@@ -669,8 +671,8 @@ __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, in
 template <typename P, int MODE, bool DAG, int REDUCE>
 __device__ __forceinline__ Sums3<typename P::real> hop_epilogue(const HopArgs& a, int rhs, int idx,
                                                                 const cplx<typename P::real> (&acc)[12]) {
-  static_assert((REDUCE != RED_DOT_SELF && REDUCE != RED_DOT_AUX) || MODE == HOP_XPAY,
-                "the dot-product reductions are fused into the XPAY epilogue");
+  static_assert((REDUCE != RED_DOT_SELF && REDUCE != RED_DOT_AUX) || MODE == HOP_XPAY || MODE == HOP_SYM,
+                "the dot-product reductions are fused into the XPAY and SYM epilogues");
   using T = typename P::real;
   cplx<T> out[12];
   cplx<T> self[12];
@@ -690,7 +692,7 @@ __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, in
   if constexpr (MODE == HOP_PLAIN) {
 #pragma unroll
     for (int k = 0; k < 12; ++k) out[k] = coef * acc[k];
-  } else if constexpr (MODE == HOP_CLOV) {
+  } else if constexpr (MODE == HOP_CLOV || MODE == HOP_SYM) {
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       T d[6];
@@ -701,6 +703,16 @@ __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, in
       clover_block_mul(y, d, o, x);
 #pragma unroll
       for (int k = 0; k < 6; ++k) out[6 * b + k] = y[k];
+    }
+    if constexpr (MODE == HOP_SYM) {
+      const char* sp = (const char*)a.self + (size_t)rhs * a.self_rhs_bytes;
+      load_spinor<P>(self, sp, a.self_norm ? a.self_norm + (size_t)rhs * a.norm_rhs_stride : nullptr, idx, g.stride);
+      const T tw = (T)(DAG ? -a.twist : a.twist);
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        out[k] = self[k] - out[k];
+        if (a.twist != 0.0) out[k] = out[k] + (k < 6 ? tw : -tw) * timesI(self[k]);
+      }
     }
   } else {  // HOP_XPAY
     const char* sp = (const char*)a.self + (size_t)rhs * a.self_rhs_bytes;

@@ -29,13 +29,15 @@ static int hop_shape(const HopArgs& a, HopShape sh, cudaStream_t s) {
   } else {
     GBC_SHAPE(128, 1, 1)
     GBC_SHAPE(128, 1, 6)
-    GBC_SHAPE(32, 4, 1)
+    if constexpr (MODE != HOP_SYM) {
+      GBC_SHAPE(32, 4, 1)
+    }
     GBC_SHAPE(32, 4, 5)
     GBC_SHAPE(64, 2, 4)
     GBC_SHAPE(32, 12, 2)
   }
 #undef GBC_SHAPE
-  if constexpr (std::is_same<P, PrecH>::value) {
+  if constexpr (std::is_same<P, PrecH>::value && MODE != HOP_SYM) {
     if (sh.pair == 3) {
       // two right-hand sides per thread: blocks of TS sites x NRB right-hand sides, TS NRB / 2 threads
       if (a.nrhs & 1) return -1;
@@ -127,6 +129,17 @@ static int hop_recon(int recon, int mode, int reduce, const HopArgs& a, HopShape
   if (recon == 12) return hop_mode<P, 12, DAG>(mode, reduce, a, sh, s);
 #endif
   return -1;
+}
+
+// the symmetric operator's second step (isign = PLUS), in translation units of its own (dslash_sym_*.cu)
+template <typename P, int RECON>
+static int hop_sym_reduce(int reduce, const HopArgs& a, HopShape sh, cudaStream_t s) {
+  switch (reduce) {
+    case RED_NONE: return hop_shape<P, RECON, HOP_SYM, false, RED_NONE>(a, sh, s);
+    case RED_NORM: return hop_shape<P, RECON, HOP_SYM, false, RED_NORM>(a, sh, s);
+    case RED_DOT_SELF: return hop_shape<P, RECON, HOP_SYM, false, RED_DOT_SELF>(a, sh, s);
+    default: return hop_shape<P, RECON, HOP_SYM, false, RED_DOT_AUX>(a, sh, s);
+  }
 }
 
 // several lattices in one launch (work table of (lattice, site block), 128-site blocks)

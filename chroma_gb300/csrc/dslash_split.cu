@@ -32,6 +32,14 @@ int launch(const HopArgs& a, int sites, cudaStream_t s) {
 
 int hop_split_launch(int mode, bool dag, int reduce, const HopArgs& a, int sites, cudaStream_t s) {
   switch (mode) {
+    case HOP_SYM:
+      if (dag) return -1;
+      switch (reduce) {
+        case RED_NONE: return launch<HOP_SYM, false, RED_NONE>(a, sites, s);
+        case RED_NORM: return launch<HOP_SYM, false, RED_NORM>(a, sites, s);
+        case RED_DOT_SELF: return launch<HOP_SYM, false, RED_DOT_SELF>(a, sites, s);
+        default: return launch<HOP_SYM, false, RED_DOT_AUX>(a, sites, s);
+      }
     case HOP_PLAIN:
       if (reduce) return -1;
       return dag ? launch<HOP_PLAIN, true, RED_NONE>(a, sites, s) : launch<HOP_PLAIN, false, RED_NONE>(a, sites, s);

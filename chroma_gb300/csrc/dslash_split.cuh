@@ -66,7 +66,8 @@ __device__ __forceinline__ double flip_if(bool neg, double v) {
 template <class A, int MODE, bool DAG, int REDUCE, int S>
 __device__ __forceinline__ void split_site(const A& f, double coef, double twist, int sblock, double (&sum)[3]) {
   __shared__ double2 uh[8][6][S];
-  __shared__ double xs[MODE == HOP_CLOV ? 24 : 1][S];
+  constexpr bool kClovOfHop = MODE == HOP_CLOV || MODE == HOP_SYM;  // the clover block acts on the hops' sum
+  __shared__ double xs[kClovOfHop ? 24 : 1][S];
   const int s = threadIdx.x % S, q = threadIdx.x / S;
   const auto& g = f.geom();
   const int idx = sblock * S + s;
@@ -138,7 +139,7 @@ __device__ __forceinline__ void split_site(const A& f, double coef, double twist
         v = hp == 0 ? x : v + x;
       }
       acc[t] = v;
-      if (MODE == HOP_CLOV) xs[r][s] = coef == 1.0 ? v : coef * v;
+      if (kClovOfHop) xs[r][s] = coef == 1.0 ? v : coef * v;
     }
   }
   double2 x[6];
@@ -150,7 +151,7 @@ __device__ __forceinline__ void split_site(const A& f, double coef, double twist
   // xs is complete; and a caller's out may be self: the site's threads have read it before any writes
   if (MODE != HOP_PLAIN) __syncthreads();
   if (!valid) return;
-  if (MODE == HOP_CLOV) {
+  if (kClovOfHop) {
 #pragma unroll
     for (int j = 0; j < 6; ++j) x[j] = make_double2(xs[12 * b + 2 * j][s], xs[12 * b + 2 * j + 1][s]);
   }
@@ -176,8 +177,14 @@ __device__ __forceinline__ void split_site(const A& f, double coef, double twist
         v = fmadd(o.x, im ? x[j].y : x[j].x, v);
         v = fmadd(flip_if(low != (im != 0), o.y), im ? x[j].x : x[j].y, v);
       }
-      if (MODE == HOP_XPAY) {
-        v = fmadd(coef, acc[t], v);
+      if (MODE == HOP_SYM) {
+        const double2 xk = f.self(c, idx, k);
+        sr = im ? xk.y : xk.x;
+        sx = im ? xk.x : xk.y;
+        v = sr - v;
+      }
+      if (MODE == HOP_XPAY) v = fmadd(coef, acc[t], v);
+      if (MODE == HOP_XPAY || MODE == HOP_SYM) {
         // + isign i mu gamma_5 self, gamma_5 = diag(1, 1, -1, -1)
         if (twist != 0.0) v += flip_if((im == 0) != (b != 0), DAG ? -twist : twist) * sx;
       }

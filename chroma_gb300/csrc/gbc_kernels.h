@@ -10,8 +10,8 @@ namespace gbc {
 void count_launch(long long n = 1);
 long long launch_count();
 
-enum { HOP_PLAIN = 0, HOP_CLOV = 1, HOP_XPAY = 2 };
-// reductions fused into the stencil epilogue: none; |out|^2; (out, self) and |out|^2 of the XPAY
+enum { HOP_PLAIN = 0, HOP_CLOV = 1, HOP_XPAY = 2, HOP_SYM = 3 };
+// reductions fused into the stencil epilogue: none; |out|^2; (out, self) and |out|^2 of the XPAY (and SYM)
 // epilogue (BiCGStab's (t, s), (t, t) for t = M~ s), three partial rows per right-hand side;
 // (aux, out) of the XPAY epilogue with aux an FP32 field (BiCGStab's (r0, v) for v = M~ p), two rows
 enum { RED_NONE = 0, RED_NORM = 1, RED_DOT_SELF = 2, RED_DOT_AUX = 3 };
@@ -84,9 +84,9 @@ struct HopArgs {
   size_t norm_rhs_stride;
   const void* gauge_fwd[4];  // links U_mu(x) of the output parity
   const void* gauge_bwd[4];  // links U_mu(x) of the input parity (used as U_mu^dag(x - mu))
-  const void* clov;          // packed clover of the output parity (HOP_CLOV, HOP_XPAY)
+  const void* clov;          // packed clover of the output parity (HOP_CLOV, HOP_XPAY, HOP_SYM)
   double a;                  // coefficient of D' psi
-  double twist;              // HOP_XPAY: twisted-mass mu (0 = none)
+  double twist;              // HOP_XPAY, HOP_SYM: twisted-mass mu (0 = none)
   double* partials;          // RED_*: sums per block, [quantity][rhs][part_stride]
   int part_stride;
   // optional per-right-hand-side flags (active[r * active_stride] != 0): a right-hand side whose
@@ -124,6 +124,11 @@ inline bool hop_shape_valid(const HopShape& sh, int prec, int nrhs, int lt) {
   if (sh.pair == 2) return prec == PREC_HALF;
   if (sh.pair == 3) return prec == PREC_HALF && nrhs % 2 == 0 && sh.nrb <= nrhs;
   return !(sh.nrb > 1 && sh.nrb > nrhs);  // a block would be mostly idle
+}
+
+// HOP_SYM (the symmetric operator's second step) is compiled for isign = PLUS and these shapes only
+inline bool hop_shape_for_mode(const HopShape& sh, int mode) {
+  return mode != HOP_SYM || (sh.pair == 0 && !(sh.tx == 32 && sh.nrb == 4 && sh.minb == 1));
 }
 
 // site blocks of one right-hand-side group (the partials each launch writes per right-hand side)
@@ -172,8 +177,10 @@ inline int hop_multi_launch(int prec, int recon, int mode, bool dag, int reduce,
 }
 
 int hop_launch_df(int recon, int mode, bool dag, int reduce, const HopArgs& a, HopShape sh, cudaStream_t s);
+int hop_sym_launch(int prec, int recon, bool dag, int reduce, const HopArgs& a, HopShape sh, cudaStream_t s);
 inline int hop_launch(int prec, int recon, int mode, bool dag, int reduce, const HopArgs& a, HopShape sh,
                       cudaStream_t s) {
+  if (mode == HOP_SYM) return hop_sym_launch(prec, recon, dag, reduce, a, sh, s);
   switch (prec) {
     case PREC_DF: return hop_launch_df(recon, mode, dag, reduce, a, sh, s);
     case PREC_DOUBLE: return hop_launch_d(recon, mode, dag, reduce, a, sh, s);
