@@ -23,6 +23,7 @@
 #include <cmath>
 #include <complex>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
 #include <random>
@@ -183,7 +184,7 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
 }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// thread 0 waits for phase `parity` of the mbarrier, for about 1 s of SM clock at most
+// waits for phase `parity` of the mbarrier, for about 1 s of SM clock at most
 __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
   const long long t0 = clock64();
   while (true) {
@@ -238,10 +239,14 @@ constexpr int kTmemCols = 32;  // tensor-memory columns allocated per block (>= 
 // columns of G are zeroed, and odd sites need only the K steps that cover the self term.
 // A block walks its tiles: weights, tensor memory and barrier are set up once, and warps 3..8 gather
 // the next tile while warps 0..2 still store this one.
+// Every thread waits for the MMA on its own clock, so a warp votes on the outcome: it uses its
+// accumulator rows (tcgen05.ld needs the whole warp) or counts one error and stores nothing.  Warp
+// `quit` (-1: none) gives up its first wait at once, for tests of that path.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int total, int batch, int per, int flags,
                                                       const float2* __restrict__ links, const float4* __restrict__ hin,
-                                                      float4* __restrict__ hout, const uint4* __restrict__ Wc) {
+                                                      float4* __restrict__ hout, const uint4* __restrict__ Wc,
+                                                      int quit) {
   constexpr int KP = kpad(CIN), NP = npad(COUT), NU = nump(COUT);
   constexpr int MROWS = 128;  // the MMA's M: the 96 rows of the tile and 32 discarded rows
   static_assert(ROWS <= MROWS && NU <= kTmemCols, "tile does not fit the MMA");
@@ -290,7 +295,7 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
     const int n = neighbour(g, par, ic, d);
     float2 m[9];
     if (mine && d > 0) load_transport(m, links, V, j, n, d);
-    if (!mine) {
+    if (!mine && ok) {
 #pragma unroll
       for (int c = 0; c < CH; ++c)
 #pragma unroll
@@ -299,10 +304,10 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
     }
     const int ksteps = (flags & IN_ODD) && par == 1 ? (2 * CIN + 15) / 16 : KP / 16;
     for (int b = b0; b < b1; ++b) {
-      if (mine) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
+      if (mine && ok) gather_dir<CIN>(G, d, s, m, hin + (size_t)b * V * planes(CIN), V, n);
       // the tensor cores read G and W through the async proxy
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      // every thread leaves together once a wait for the previous MMA has given up
+      // every thread leaves together once a warp's wait for the previous MMA has given up
       if (!__syncthreads_and(ok)) {
         dead = true;
         break;
@@ -325,9 +330,9 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
       }
       // every thread waits: the MMA has read G (the next gather may overwrite it) and written its
       // accumulators
-      ok = mbar_wait(smem_u32(&mbar), phase);
+      ok = __all_sync(0xffffffffu, d != quit && mbar_wait(smem_u32(&mbar), phase));
       if (!ok) {
-        if (tid == 0) atomicAdd(&g_tc_wait_errors, 1);
+        if (s == 0) atomicAdd(&g_tc_wait_errors, 1);
         // give the MMAs in flight one more bounded wait before their tensor memory is freed
         (void)mbar_wait(smem_u32(&mbar), phase);
       }
@@ -621,7 +626,7 @@ Split split_of(const Geom& g, int batch, int flags) {
 
 template <int CIN, int COUT>
 void launch_layer(const Geom& g, int V, int batch, int flags, const float2* links, const float4* in, float4* out,
-                  const __nv_bfloat16* W, cudaStream_t s) {
+                  const __nv_bfloat16* W, int quit, cudaStream_t s) {
   // G (96 rows) and W (npad rows) in the core-matrix layout, inside the 128 rows x kpad that the
   // MMA's A operand (and its B operand, ending at the same row) spans
   const size_t smem = (size_t)128 * kpad(CIN) * 2;
@@ -629,7 +634,7 @@ void launch_layer(const Geom& g, int V, int batch, int flags, const float2* link
   const Split w = split_of(g, batch, flags);
   // three resident blocks per SM
   layer_kernel<CIN, COUT><<<dim3(std::min(w.blocks, 3 * 152), w.parts), CT, smem, s>>>(
-      g, V, w.tiles, w.blocks, batch, w.per, flags, links, in, out, reinterpret_cast<const uint4*>(W));
+      g, V, w.tiles, w.blocks, batch, w.per, flags, links, in, out, reinterpret_cast<const uint4*>(W), quit);
   count_launch();
 }
 
@@ -648,11 +653,11 @@ void launch_wgrad(const Geom& g, int V, int batch, int flags, const float2* link
 }
 
 void layer(const Geom& g, int V, int batch, int cin, int cout, int flags, const float2* links, const float4* in,
-           float4* out, const __nv_bfloat16* W, cudaStream_t s) {
-  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, flags, links, in, out, W, s);
-  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, flags, links, in, out, W, s);
-  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, flags, links, in, out, W, s);
-  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, flags, links, in, out, W, s);
+           float4* out, const __nv_bfloat16* W, int quit, cudaStream_t s) {
+  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, flags, links, in, out, W, quit, s);
+  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, flags, links, in, out, W, quit, s);
+  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, flags, links, in, out, W, quit, s);
+  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, flags, links, in, out, W, quit, s);
   else throw std::string("network layer shape not compiled");
 }
 
@@ -700,6 +705,9 @@ void Cnn::init(int hidden_, int layers_, unsigned long long seed) {
   }
   step = 0;
   dirty = true;
+  // GBC_TC_QUIT_WARP=<warp>: that warp of every layer block gives up its waits (error-path tests)
+  const char* q = getenv("GBC_TC_QUIT_WARP");
+  quit = q && *q ? atoi(q) : -1;
 }
 
 // Real form of a layer's weights in the MMA's order (comp) and core-matrix layout: rows n = comp(o, .)
@@ -811,7 +819,7 @@ void Cnn::forward(gbc_ctx* c, int batch) {
   const int V = (int)c->V;
   for (int l = 0; l < nlayers; ++l)
     layer(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (l == nlayers - 1 ? OUT_ODD : 0), links, act[l],
-          act[l + 1], dW[l], c->stream);
+          act[l + 1], dW[l], quit, c->stream);
 }
 
 // A layer whose wait for its tensor-core results gave up (it then frees its tensor memory and
@@ -843,7 +851,7 @@ double Cnn::loss_and_grad(gbc_ctx* c, int batch) {
     wgrad(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (last ? OUT_ODD : 0), links, act[l], delta[cur],
           dG + grad_offset(l), s);
     if (l > 0) {
-      layer(c->g, V, batch, cout(l), cin(l), last ? IN_ODD : 0, links, delta[cur], delta[1 - cur], dWadj[l], s);
+      layer(c->g, V, batch, cout(l), cin(l), last ? IN_ODD : 0, links, delta[cur], delta[1 - cur], dWadj[l], quit, s);
       cur = 1 - cur;
     }
   }

@@ -22,6 +22,7 @@ struct Cnn {
   std::vector<std::vector<float>> m1, m2;  // Adam moments (re, im interleaved)
   long step = 0;
   bool dirty = true;
+  int quit = -1;  // warp whose waits for the tensor cores give up at once (-1: none)
 
   __nv_bfloat16* dW[8] = {nullptr};     // real form, npad(cout) x kpad(cin) in core-matrix layout
   __nv_bfloat16* dWadj[8] = {nullptr};  // input-gradient form
