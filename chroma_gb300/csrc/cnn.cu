@@ -170,8 +170,6 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 // (NU rows = output channels x re/im, padded to a multiple of 16); completion is signalled through
 // an mbarrier by tcgen05.commit, and each warp reads its 32 accumulator lanes back with tcgen05.ld.
 
-__device__ int g_tc_wait_errors;  // waits for tensor-core completion that gave up (host-checked)
-
 // shared-memory matrix descriptor, K-major without swizzle: start, leading byte offset (between
 // K-adjacent core matrices), stride byte offset (between 8-row groups), descriptor version 1
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
@@ -240,13 +238,14 @@ constexpr int kTmemCols = 32;  // tensor-memory columns allocated per block (>= 
 // A block walks its tiles: weights, tensor memory and barrier are set up once, and warps 3..8 gather
 // the next tile while warps 0..2 still store this one.
 // Every thread waits for the MMA on its own clock, so a warp votes on the outcome: it uses its
-// accumulator rows (tcgen05.ld needs the whole warp) or counts one error and stores nothing.  Warp
+// accumulator rows (tcgen05.ld needs the whole warp) or counts one error (its network's, read by the
+// host) and stores nothing.  Warp
 // `quit` (-1: none) gives up its first wait at once, for tests of that path.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int total, int batch, int per, int flags,
                                                       const float2* __restrict__ links, const float4* __restrict__ hin,
                                                       float4* __restrict__ hout, const uint4* __restrict__ Wc,
-                                                      int quit) {
+                                                      int* errors, int quit) {
   constexpr int KP = kpad(CIN), NP = npad(COUT), NU = nump(COUT);
   constexpr int MROWS = 128;  // the MMA's M: the 96 rows of the tile and 32 discarded rows
   static_assert(ROWS <= MROWS && NU <= kTmemCols, "tile does not fit the MMA");
@@ -332,7 +331,7 @@ __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, 
       // accumulators
       ok = __all_sync(0xffffffffu, d != quit && mbar_wait(smem_u32(&mbar), phase));
       if (!ok) {
-        if (s == 0) atomicAdd(&g_tc_wait_errors, 1);
+        if (s == 0) atomicAdd(errors, 1);
         // give the MMAs in flight one more bounded wait before their tensor memory is freed
         (void)mbar_wait(smem_u32(&mbar), phase);
       }
@@ -626,7 +625,7 @@ Split split_of(const Geom& g, int batch, int flags) {
 
 template <int CIN, int COUT>
 void launch_layer(const Geom& g, int V, int batch, int flags, const float2* links, const float4* in, float4* out,
-                  const __nv_bfloat16* W, int quit, cudaStream_t s) {
+                  const __nv_bfloat16* W, int* errors, int quit, cudaStream_t s) {
   // G (96 rows) and W (npad rows) in the core-matrix layout, inside the 128 rows x kpad that the
   // MMA's A operand (and its B operand, ending at the same row) spans
   const size_t smem = (size_t)128 * kpad(CIN) * 2;
@@ -634,7 +633,7 @@ void launch_layer(const Geom& g, int V, int batch, int flags, const float2* link
   const Split w = split_of(g, batch, flags);
   // three resident blocks per SM
   layer_kernel<CIN, COUT><<<dim3(std::min(w.blocks, 3 * 152), w.parts), CT, smem, s>>>(
-      g, V, w.tiles, w.blocks, batch, w.per, flags, links, in, out, reinterpret_cast<const uint4*>(W), quit);
+      g, V, w.tiles, w.blocks, batch, w.per, flags, links, in, out, reinterpret_cast<const uint4*>(W), errors, quit);
   count_launch();
 }
 
@@ -653,11 +652,11 @@ void launch_wgrad(const Geom& g, int V, int batch, int flags, const float2* link
 }
 
 void layer(const Geom& g, int V, int batch, int cin, int cout, int flags, const float2* links, const float4* in,
-           float4* out, const __nv_bfloat16* W, int quit, cudaStream_t s) {
-  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, flags, links, in, out, W, quit, s);
-  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, flags, links, in, out, W, quit, s);
-  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, flags, links, in, out, W, quit, s);
-  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, flags, links, in, out, W, quit, s);
+           float4* out, const __nv_bfloat16* W, int* errors, int quit, cudaStream_t s) {
+  if (cin == 4 && cout == 12) launch_layer<4, 12>(g, V, batch, flags, links, in, out, W, errors, quit, s);
+  else if (cin == 12 && cout == 12) launch_layer<12, 12>(g, V, batch, flags, links, in, out, W, errors, quit, s);
+  else if (cin == 12 && cout == 4) launch_layer<12, 4>(g, V, batch, flags, links, in, out, W, errors, quit, s);
+  else if (cin == 4 && cout == 4) launch_layer<4, 4>(g, V, batch, flags, links, in, out, W, errors, quit, s);
   else throw std::string("network layer shape not compiled");
 }
 
@@ -759,17 +758,22 @@ void Cnn::release() {
   }
   for (auto& p : act) if (p) cudaFree(p);
   act.clear();
-  for (void* p : {(void*)links, (void*)delta[0], (void*)delta[1], (void*)target, (void*)dG, (void*)norms})
+  for (void* p : {(void*)links, (void*)delta[0], (void*)delta[1], (void*)target, (void*)dG, (void*)norms, (void*)errors})
     if (p) cudaFree(p);
   links = nullptr;
   delta[0] = delta[1] = target = nullptr;
   dG = nullptr;
   norms = nullptr;
+  errors = nullptr;
   act_batch = train_batch = 0;
 }
 
 void Cnn::ensure(gbc_ctx* c, int batch) {
   const int V = (int)c->V;
+  if (!errors) {
+    GBC_CUDA(cudaMalloc(&errors, sizeof(int)));
+    GBC_CUDA(cudaMemsetAsync(errors, 0, sizeof(int), c->stream));
+  }
   if (!links || links_version != c->gauge_version) {
     if (!links) GBC_CUDA(cudaMalloc(&links, sizeof(float2) * (size_t)V * 36));
     links_kernel<<<(V + 127) / 128, 128, 0, c->stream>>>(c->g, V, reinterpret_cast<const double2*>(c->d_links), links);
@@ -819,18 +823,18 @@ void Cnn::forward(gbc_ctx* c, int batch) {
   const int V = (int)c->V;
   for (int l = 0; l < nlayers; ++l)
     layer(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (l == nlayers - 1 ? OUT_ODD : 0), links, act[l],
-          act[l + 1], dW[l], quit, c->stream);
+          act[l + 1], dW[l], errors, quit, c->stream);
 }
 
 // A layer whose wait for its tensor-core results gave up (it then frees its tensor memory and
-// returns) counts in g_tc_wait_errors: read and reset it, and fail the call that ran the layers.
-void cnn_check_waits(cudaStream_t s) {
+// returns) counts in `errors`: read and reset it, and fail the call that ran the layers.
+void Cnn::check_waits(cudaStream_t s) {
+  if (!errors) return;  // no layer has run
   int n = 0;
-  GBC_CUDA(cudaMemcpyFromSymbolAsync(&n, g_tc_wait_errors, sizeof(int), 0, cudaMemcpyDeviceToHost, s));
+  GBC_CUDA(cudaMemcpyAsync(&n, errors, sizeof(int), cudaMemcpyDeviceToHost, s));
   GBC_CUDA(cudaStreamSynchronize(s));
   if (n) {
-    const int zero = 0;
-    GBC_CUDA(cudaMemcpyToSymbol(g_tc_wait_errors, &zero, sizeof(int)));
+    GBC_CUDA(cudaMemsetAsync(errors, 0, sizeof(int), s));
     throw std::string("network layer: a wait for the tensor cores gave up");
   }
 }
@@ -851,13 +855,13 @@ double Cnn::loss_and_grad(gbc_ctx* c, int batch) {
     wgrad(c->g, V, batch, cin(l), cout(l), (l == 0 ? IN_ODD : 0) | (last ? OUT_ODD : 0), links, act[l], delta[cur],
           dG + grad_offset(l), s);
     if (l > 0) {
-      layer(c->g, V, batch, cout(l), cin(l), last ? IN_ODD : 0, links, delta[cur], delta[1 - cur], dWadj[l], quit, s);
+      layer(c->g, V, batch, cout(l), cin(l), last ? IN_ODD : 0, links, delta[cur], delta[1 - cur], dWadj[l], errors, quit, s);
       cur = 1 - cur;
     }
   }
   double loss = 0;
   GBC_CUDA(cudaMemcpyAsync(&loss, dl, sizeof(double), cudaMemcpyDeviceToHost, s));
-  cnn_check_waits(s);
+  check_waits(s);
   return loss;
 }
 

@@ -31,6 +31,7 @@ struct Cnn {
   float4* delta[2] = {nullptr, nullptr};
   float4* target = nullptr;             // training targets, as 4-channel activations
   double* norms = nullptr;              // |target_b|^2, then the loss
+  int* errors = nullptr;                // waits for the tensor cores that gave up since the last check
   int act_batch = 0, train_batch = 0;
   float2* links = nullptr;              // FP32 links, planes [4 * 9][V] in even-odd order
   long links_version = -1;
@@ -50,13 +51,13 @@ struct Cnn {
   void adam(const std::vector<std::vector<std::complex<float>>>& grad, double lr);
   bool save(const std::string& path) const;
   int load(const std::string& path);
+  // waits for the stream and throws if a layer gave up waiting for the tensor cores since the last check
+  void check_waits(cudaStream_t s);
   void release();
 };
 
-// (the caller runs cnn_check_waits before it relies on the result)
+// (the caller runs net.check_waits before it relies on the result)
 void cnn_apply_spinor(gbc_ctx* c, Cnn& net, const Spinor& in, const Spinor& out);
-// waits for the stream and throws if a layer gave up waiting for the tensor cores since the last check
-void cnn_check_waits(cudaStream_t s);
 // norm2 (may be null): |f_b|^2 of each field over the odd sites, summed in FP64
 void cnn_embed_canon(gbc_ctx* c, Cnn& net, int batch, const double* canon_dev, float4* act, double* norm2 = nullptr);
 void cnn_extract_canon(gbc_ctx* c, Cnn& net, int batch, const float4* act, double* canon_dev);

@@ -32,7 +32,7 @@ void precond_apply(gbc_ctx* c, const Spinor& in, const Spinor& out) {
 }
 
 void precond_check(gbc_ctx* c) {
-  if (c->precond) cnn_check_waits(c->stream);
+  if (c->precond) net_of(c)->check_waits(c->stream);
 }
 
 int precond_layers(gbc_ctx* c) { return c->precond ? net_of(c)->nlayers : 0; }
@@ -139,7 +139,7 @@ int gbc_precond_apply(gbc_ctx* c, int nrhs, double* out, const double* in) {
     cnn_embed_canon(c, n, nrhs, c->d_stage[0], n.act[0]);
     n.forward(c, nrhs);
     cnn_extract_canon(c, n, nrhs, n.act[n.nlayers], c->d_stage[1]);
-    cnn_check_waits(c->stream);
+    n.check_waits(c->stream);
     res.send(0);
     res.wait();
     sync(c);

@@ -3,6 +3,8 @@ the warp that issues the MMA (0), one that only stores (2), one that only gather
 the waits of one warp give up at once; the block then waits for its MMA all the same and leaves.
 
 Exact: a call either fails, or its result is the one of an undisturbed network."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -40,3 +42,39 @@ def test_given_up_wait_fails_the_call(dims, nrhs, warp, monkeypatch):
         assert np.array_equal(ctx.precond_apply(x), want)
     finally:
         ctx.close()
+
+
+def test_contexts_count_their_own_waits(monkeypatch):
+    """Two contexts on two threads, the waits of one giving up: each of its calls fails, none of the other's."""
+    dims, calls = (8, 8, 8, 8), 40
+    x = S.gaussian(dims, 3, cb=1).reshape(1, -1, 12).astype(np.complex128)
+    bad, good = _context(dims), _context(dims)
+    try:
+        good.precond_init(hidden=12, layers=3, seed=1)
+        want = good.precond_apply(x)
+        monkeypatch.setenv("GBC_TC_QUIT_WARP", "0")
+        bad.precond_init(hidden=12, layers=3, seed=1)
+        monkeypatch.delenv("GBC_TC_QUIT_WARP")
+        failed, right = [], []
+
+        def run(ctx, start):
+            start.wait()
+            for _ in range(calls):
+                try:
+                    y = ctx.precond_apply(x)
+                    if ctx is good:
+                        right.append(np.array_equal(y, want))
+                except G.GBCError:
+                    failed.append(ctx)
+
+        start = threading.Barrier(2)
+        threads = [threading.Thread(target=run, args=(ctx, start)) for ctx in (bad, good)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert failed == [bad] * calls
+        assert right == [True] * calls
+    finally:
+        bad.close()
+        good.close()
