@@ -325,10 +325,23 @@ int solve_multishift(gbc_ctx* c, const gbc_solve_params* pp, int ns, const doubl
       double* d_shift = nullptr;
       GBC_CUDA(cudaMalloc(&d_shift, sizeof(double) * ns));
       GBC_CUDA(cudaMemcpyAsync(d_shift, shift.data(), sizeof(double) * ns, cudaMemcpyHostToDevice, s));
-      std::vector<double> rsdv(rsd, rsd + ns);
+      refine_rr.resize(ns);
+      rr_final = true;
       try {
-        refine_iters = refine_shifted(c, sp, chid, d_shift, XD, rsdv, std::max(1, max_iter - iters), refine_rr,
-                                      refine_status, rr_final);
+        // the context's scalars and partial sums are sized for max_rhs right-hand sides
+        for (int q0 = 0; q0 < ns; q0 += c->max_rhs) {
+          const int m = std::min(c->max_rhs, ns - q0);
+          std::vector<double> rr;
+          std::vector<int> st;
+          bool last = false;
+          const std::vector<int> it = refine_shifted(c, sp, chid, d_shift + q0, sub(XD, q0, m),
+                                                     std::vector<double>(rsd + q0, rsd + q0 + m),
+                                                     std::max(1, max_iter - iters), rr, st, last);
+          std::copy(it.begin(), it.end(), refine_iters.begin() + q0);
+          std::copy(st.begin(), st.end(), refine_status.begin() + q0);
+          std::copy(rr.begin(), rr.end(), refine_rr.begin() + q0);
+          rr_final = rr_final && last;
+        }
       } catch (...) {
         cudaFree(d_shift);
         throw;

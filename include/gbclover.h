@@ -313,7 +313,8 @@ int gbc_gauge_synthetic(const int dims[4], double eps, unsigned long long seed, 
    corrections from CG on the shifted system in the sloppy operator (n_count adds those iterations);
    0 or GBC_PREC_DOUBLE runs the recursion in FP64 to the targets.  chi and every psi[s]
    are canonical host arrays (only their odd sites are read / written); res[s] per shift, with the
-   FP64 true relative residual of that shifted system. */
+   FP64 true relative residual of that shifted system.  max_rhs does not limit nshift: the mixed
+   form refines the shifts in groups of max_rhs. */
 int gbc_solve_multishift(gbc_ctx* ctx, const gbc_solve_params* p, int nshift, const double* shifts,
                          const double* rsd_targets, double* const* psi, const double* chi, gbc_result* res);
 
