@@ -45,36 +45,41 @@ def test_given_up_wait_fails_the_call(dims, nrhs, warp, monkeypatch):
 
 
 def test_contexts_count_their_own_waits(monkeypatch):
-    """Two contexts on two threads, the waits of one giving up: each of its calls fails, none of the other's."""
-    dims, calls = (8, 8, 8, 8), 40
-    x = S.gaussian(dims, 3, cb=1).reshape(1, -1, 12).astype(np.complex128)
-    bad, good = _context(dims), _context(dims)
+    """Two contexts on two threads, the waits of one giving up: each of its calls fails, and none of the calls
+    that the other makes meanwhile."""
+    x = S.gaussian((8, 8, 8, 8), 3, cb=1).reshape(1, -1, 12).astype(np.complex128)
+    y = S.gaussian((16, 16, 16, 16), 3, cb=1).reshape(1, -1, 12).astype(np.complex128)
+    bad, good = _context((16, 16, 16, 16)), _context((8, 8, 8, 8))
     try:
-        good.precond_init(hidden=12, layers=3, seed=1)
+        good.precond_init(hidden=12, layers=2, seed=1)
         want = good.precond_apply(x)
         monkeypatch.setenv("GBC_TC_QUIT_WARP", "0")
-        bad.precond_init(hidden=12, layers=3, seed=1)
+        bad.precond_init(hidden=12, layers=8, seed=1)
         monkeypatch.delenv("GBC_TC_QUIT_WARP")
-        failed, right = [], []
+        failed, right, done = [], [], threading.Event()
 
-        def run(ctx, start):
-            start.wait()
-            for _ in range(calls):
+        def fails():
+            for _ in range(100):
                 try:
-                    y = ctx.precond_apply(x)
-                    if ctx is good:
-                        right.append(np.array_equal(y, want))
+                    bad.precond_apply(y)
+                    failed.append(False)
                 except G.GBCError:
-                    failed.append(ctx)
+                    failed.append(True)
+            done.set()
 
-        start = threading.Barrier(2)
-        threads = [threading.Thread(target=run, args=(ctx, start)) for ctx in (bad, good)]
+        def works():
+            while not done.is_set():
+                try:
+                    right.append(np.array_equal(good.precond_apply(x), want))
+                except G.GBCError:
+                    right.append(False)
+
+        threads = [threading.Thread(target=f) for f in (fails, works)]
         for t in threads:
             t.start()
         for t in threads:
             t.join()
-        assert failed == [bad] * calls
-        assert right == [True] * calls
+        assert all(failed) and all(right) and len(right) > 1
     finally:
         bad.close()
         good.close()
