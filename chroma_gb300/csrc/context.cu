@@ -282,21 +282,55 @@ static int default_shape(int prec, int nrhs) {
   return 1;
 }
 
+// one line of the tune report: a decision and where it came from
+static void log_shape(gbc_ctx* c, int prec, int mode, bool dag, int reduce, int nrhs, int si, const char* origin) {
+  const HopShape& sh = kHopShapes[si];
+  char line[160];
+  snprintf(line, sizeof line, "prec=%d mode=%d dag=%d reduce=%d nrhs=%d -> tx=%d nrb=%d minb=%d pair=%d (%s)\n", prec,
+           mode, dag ? 1 : 0, reduce, nrhs, sh.tx, sh.nrb, sh.minb, sh.pair, origin);
+  c->tune_log += line;
+}
+
+// (precision, epilogue, isign, reduction) in the high bits, nrhs (any size) in the low 32
+static long long shape_key(int prec, int mode, bool dag, int reduce, int nrhs) {
+  return ((((long long)pidx(prec) * 4 + mode) * 2 + (dag ? 1 : 0)) * 4 + reduce) << 32 | (unsigned)nrhs;
+}
+
+// GBC_SHAPE=<index into kHopShapes> pins one shape (profiling, tests of a kernel); -1: none, or not one
+// that this launch can take
+static int pinned_shape(int prec, int mode, const HopArgs& h) {
+  const char* fs = getenv("GBC_SHAPE");
+  if (!fs) return -1;
+  const int si = atoi(fs);
+  const bool ok = si >= 0 && si < kNumHopShapes && hop_shape_valid(kHopShapes[si], prec, h.nrhs, h.g.L[3]) &&
+                  hop_shape_for_mode(kHopShapes[si], mode);
+  return ok ? si : -1;
+}
+
+// Whether an FP64 launch runs on the split kernel: by its size (hop_split), unless a shape of hop_kernel
+// is pinned.  Decided once per kind of launch and kept in c->tuned, as tuned_shape's choices (kSplit).
+constexpr int kSplit = -1;
+static bool use_split(gbc_ctx* c, int prec, int mode, bool dag, int reduce, const HopArgs& h) {
+  if (prec != PREC_DOUBLE || !hop_split(h.g.Vh, h.nrhs)) return false;
+  const long long key = shape_key(prec, mode, dag, reduce, h.nrhs);
+  auto it = c->tuned.find(key);
+  if (it == c->tuned.end()) {
+    const int si = pinned_shape(prec, mode, h);
+    it = c->tuned.emplace(key, si < 0 ? kSplit : si).first;
+    if (si >= 0) log_shape(c, prec, mode, dag, reduce, h.nrhs, si, "GBC_SHAPE");
+  }
+  return it->second == kSplit;
+}
+
 int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce, const HopArgs& h) {
-  // (precision, epilogue, isign, reduction) in the high bits, nrhs (any size) in the low 32
-  const long long key =
-      ((((long long)pidx(prec) * 4 + mode) * 2 + (dag ? 1 : 0)) * 4 + reduce) << 32 | (unsigned)h.nrhs;
+  const long long key = shape_key(prec, mode, dag, reduce, h.nrhs);
   auto it = c->tuned.find(key);
   if (it != c->tuned.end()) return it->second;
   int best = default_shape(prec, h.nrhs);
-  // GBC_SHAPE=<index into kHopShapes> pins one shape (profiling); ignored when out of range
-  if (const char* fs = getenv("GBC_SHAPE")) {
-    const int si = atoi(fs);
-    if (si >= 0 && si < kNumHopShapes && hop_shape_valid(kHopShapes[si], prec, h.nrhs, h.g.L[3]) &&
-        hop_shape_for_mode(kHopShapes[si], mode)) {
-      c->tuned[key] = si;
-      return si;
-    }
+  if (const int si = pinned_shape(prec, mode, h); si >= 0) {
+    log_shape(c, prec, mode, dag, reduce, h.nrhs, si, "GBC_SHAPE");
+    c->tuned[key] = si;
+    return si;
   }
   const char* cpath = getenv("GBC_TUNE_CACHE");
   const bool cached = c->autotune && cpath && *cpath;
@@ -336,10 +370,7 @@ int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce,
         if (sh.tx == t[0] && sh.nrb == t[1] && sh.minb == t[2] && sh.pair == t[3] &&
             hop_shape_valid(sh, prec, h.nrhs, h.g.L[3]) && hop_shape_for_mode(sh, mode) &&
             hop_blocks(sh, h.g.Vh) <= h.part_stride) {
-          char line[160];
-          snprintf(line, sizeof line, "prec=%d mode=%d dag=%d reduce=%d nrhs=%d -> tx=%d nrb=%d minb=%d pair=%d (%s)\n",
-                   prec, mode, dag ? 1 : 0, reduce, h.nrhs, sh.tx, sh.nrb, sh.minb, sh.pair, origin);
-          c->tune_log += line;
+          log_shape(c, prec, mode, dag, reduce, h.nrhs, si, origin);
           c->tuned[key] = si;
           return si;
         }
@@ -388,11 +419,9 @@ int tuned_shape(gbc_ctx* c, int prec, int recon, int mode, bool dag, int reduce,
     count_launch(launches);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    char line[160];
-    snprintf(line, sizeof line, "prec=%d mode=%d dag=%d reduce=%d nrhs=%d -> tx=%d nrb=%d minb=%d pair=%d (%.1f us)\n",
-             prec, mode, dag ? 1 : 0, reduce, h.nrhs, kHopShapes[best].tx, kHopShapes[best].nrb,
-             kHopShapes[best].minb, kHopShapes[best].pair, best_ms * 1e3);
-    c->tune_log += line;
+    char us[32];
+    snprintf(us, sizeof us, "%.1f us", best_ms * 1e3);
+    log_shape(c, prec, mode, dag, reduce, h.nrhs, best, us);
     if (cached) {
       const HopShape& sh = kHopShapes[best];
       TuneCache& tc = tune_cache();
@@ -470,7 +499,7 @@ void hop(gbc_ctx* c, int prec, int out_parity, int mode, bool dag, double a, con
     finished = reduce && one_rhs && finish_in_kernel((long)blocks * h.nrhs);
     if (finished) h.fin = sums.finish();
   };
-  if (prec == PREC_DOUBLE && hop_split(h.g.Vh, h.nrhs)) {
+  if (use_split(c, prec, mode, dag, reduce, h)) {
     const int sites = hop_split_sites(h.g.Vh, h.nrhs);
     set_finish((h.g.Vh + sites - 1) / sites, true);
     nb = hop_split_launch(mode, dag, reduce, h, sites, c->stream);
