@@ -32,41 +32,29 @@ size_t total_bytes(const PageTouch::Ranges& ranges) {
 
 }  // namespace
 
-void PageTouch::populate(Ranges ranges, std::function<void()> then) {
+void PageTouch::populate(Ranges ranges, std::function<void()> then, int threads) {
   join();
   then_ = std::move(then);
-  if (total_bytes(ranges) < kSmall) return;
-  try {
-    th_[0] = std::thread([this, ranges = std::move(ranges), page = page_size()] {
-      for (const auto& r : ranges) {
-        const uintptr_t p = reinterpret_cast<uintptr_t>(r.first) & ~(uintptr_t)(page - 1);
-        const uintptr_t end = reinterpret_cast<uintptr_t>(r.first) + r.second;
-        (void)madvise(reinterpret_cast<void*>(p), end - p, MADV_POPULATE_WRITE);
-      }
-      if (then_) then_();
-      then_ = nullptr;
-    });
-  } catch (const std::exception&) {  // no thread: join() runs `then`
-  }
-}
-
-void PageTouch::overwrite(Ranges ranges) {
-  join();
-  const size_t total = total_bytes(ranges), page = page_size();
+  const size_t total = total_bytes(ranges);
   if (total < kSmall) return;
-  const int cores = (int)std::max(1u, std::thread::hardware_concurrency());
-  // one thread per 8 MB, up to 8 (16 were no faster) and half of the cores
-  const int n = (int)std::min<size_t>(std::min(8, std::max(1, cores / 2)), total / (8u << 20) + 1);
+  // one per 8 MB: a helper takes some 50 us to start
+  const int n = std::min({std::max(threads, 1), (int)kThreads, (int)std::min<size_t>(total / (8u << 20) + 1, kThreads)});
+  left_ = n;
   try {
     for (int k = 0; k < n; ++k)
-      th_[k] = std::thread([ranges, page, k, n] {
+      th_[k] = std::thread([this, ranges, page = page_size(), k, n] {
         for (const auto& r : ranges) {
-          volatile char* p = static_cast<volatile char*>(r.first);
-          const size_t pages = (r.second + page - 1) / page;
-          for (size_t i = pages * k / n; i < pages * (k + 1) / n; ++i) p[i * page] = 0;
+          const uintptr_t base = reinterpret_cast<uintptr_t>(r.first);
+          const uintptr_t p = (base + r.second / n * k) & ~(uintptr_t)(page - 1);
+          const uintptr_t end = base + (k + 1 == n ? r.second : r.second / n * (k + 1));
+          if (end > p) (void)madvise(reinterpret_cast<void*>(p), end - p, MADV_POPULATE_WRITE);
+        }
+        if (left_.fetch_sub(1) == 1 && then_) {
+          then_();
+          then_ = nullptr;
         }
       });
-  } catch (const std::exception&) {
+  } catch (const std::exception&) {  // no thread: join() runs `then`
   }
 }
 
@@ -77,16 +65,14 @@ void PageTouch::join() {
   then_ = nullptr;
 }
 
-HostResult::HostResult(cudaStream_t work, cudaStream_t copy, std::vector<Item> items, Mode mode)
+HostResult::HostResult(cudaStream_t work, cudaStream_t copy, std::vector<Item> items, Mode mode, int threads)
     : work_(work), copy_(copy), items_(std::move(items)), load_(mode == kLoad) {
   GBC_CUDA(cudaGetDevice(&dev_));
   GBC_CUDA(cudaEventCreateWithFlags(&ev_, cudaEventDisableTiming));
   PageTouch::Ranges ranges;
   for (const Item& i : items_) ranges.push_back({i.host, i.bytes});
-  if (mode == kWhole) {
-    touch_.overwrite(std::move(ranges));
-  } else if (mode == kKeep) {
-    touch_.populate(std::move(ranges));
+  if (mode == kKeep) {
+    touch_.populate(std::move(ranges), nullptr, threads);
   } else {
     // the slots may still be in use by work enqueued before this call
     GBC_CUDA(cudaEventRecord(ev_, work_));
@@ -95,7 +81,7 @@ HostResult::HostResult(cudaStream_t work, cudaStream_t copy, std::vector<Item> i
       err_ = cudaSetDevice(dev_);
       for (const Item& i : items_)
         if (err_ == cudaSuccess) err_ = cudaMemcpyAsync(i.dev, i.host, i.bytes, cudaMemcpyHostToDevice, copy_);
-    });
+    }, threads);
   }
 }
 

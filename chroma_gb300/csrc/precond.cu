@@ -132,8 +132,7 @@ int gbc_precond_apply(gbc_ctx* c, int nrhs, double* out, const double* in) {
     Cnn& n = *net_of(c);
     ensure_stage(c, nrhs);
     const size_t bytes = (size_t)nrhs * c->V * 24 * sizeof(double);
-    HostResult res(c->stream, copy_stream(c), {{out, c->d_stage[1], bytes}},
-                   overlap(out, in, bytes) ? HostResult::kKeep : HostResult::kWhole);
+    HostResult res(c->stream, copy_stream(c), {{out, c->d_stage[1], bytes}}, HostResult::kKeep, PageTouch::kThreads);
     GBC_CUDA(cudaMemcpyAsync(c->d_stage[0], in, bytes, cudaMemcpyHostToDevice, c->stream));
     n.ensure(c, nrhs);
     cnn_embed_canon(c, n, nrhs, c->d_stage[0], n.act[0]);

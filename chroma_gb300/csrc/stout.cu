@@ -224,14 +224,14 @@ extern "C" int gbc_stout_smear(const gbc_geom* geom, int n_steps, double rho, co
   cudaStream_t s = nullptr;
   int rc = GBC_OK;
   PageTouch touch;
-  try {
-    if (!overlap(links_out, links_in, bytes)) touch.overwrite({{links_out, bytes}});
-  } catch (...) {  // no host memory for the helpers: the copy meets the page faults itself
-  }
   if (cudaMalloc(&buf[0], bytes) != cudaSuccess || cudaMalloc(&buf[1], bytes) != cudaSuccess ||
       cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
     rc = GBC_ERR_CUDA;
   } else {
+    try {
+      touch.populate({{links_out, bytes}}, nullptr, PageTouch::kThreads);
+    } catch (...) {  // no host memory for the helpers: the copy meets the page faults itself
+    }
     cudaMemcpyAsync(buf[0], links_in, bytes, cudaMemcpyHostToDevice, s);
     for (int i = 0; i < n_steps; ++i) {
       stout_kernel<<<(unsigned)((g.V + 31) / 32), 128, 0, s>>>(g, buf[i & 1], buf[(i + 1) & 1], rho, dirs);
