@@ -32,6 +32,15 @@ size_t total_bytes(const PageTouch::Ranges& ranges) {
 
 }  // namespace
 
+bool pages_present(const void* p, size_t bytes) {
+  const size_t page = page_size();
+  const uintptr_t lo = reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)(page - 1);
+  const size_t len = reinterpret_cast<uintptr_t>(p) + bytes - lo;
+  std::vector<unsigned char> in((len + page - 1) / page);
+  if (mincore(reinterpret_cast<void*>(lo), len, in.data()) != 0) return false;
+  return std::all_of(in.begin(), in.end(), [](unsigned char b) { return b & 1; });
+}
+
 void PageTouch::populate(Ranges ranges, std::function<void()> then, int threads) {
   join();
   then_ = std::move(then);

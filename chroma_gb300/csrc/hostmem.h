@@ -38,6 +38,9 @@ class PageTouch {
   std::function<void()> then_;
 };
 
+// whether every page of a buffer is there (25 us for 302 MB); a page that was only read counts too
+bool pages_present(const void* p, size_t bytes);
+
 // The results of a call on their way to the caller's buffers, whose pages are made resident meanwhile.
 //   kKeep  the device slots hold whatever the call puts there (the whole result, or a buffer that the
 //          caller fetched itself)
