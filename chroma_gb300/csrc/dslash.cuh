@@ -617,12 +617,19 @@ __device__ __forceinline__ Sums3<T> operator+(Sums3<T> a, const Sums3<T>& b) {
   return a;
 }
 
+// the epilogue's operands at one site, where the kernel has fetched them itself (fp16 storage)
+struct HeldSite {
+  HalfSite self;
+  cplx<float> aux[12];
+};
+
 // Store one output site in the output precision and return its site sums of the REDUCE kind
-// (self: the XPAY operand, for RED_DOT_SELF).
+// (self: the XPAY operand, for RED_DOT_SELF; aux: the FP32 field at the site, for RED_DOT_AUX).
 template <typename P, int REDUCE>
 __device__ __forceinline__ Sums3<typename P::real> store_site(const HopArgs& a, int rhs, int idx,
                                                               const cplx<typename P::real> (&out)[12],
-                                                              const cplx<typename P::real> (&self)[12]) {
+                                                              const cplx<typename P::real> (&self)[12],
+                                                              const cplx<float> (&aux)[12]) {
   using T = typename P::real;
   char* op = (char*)a.out + (size_t)rhs * a.out_rhs_bytes;
   store_spinor<P>(op, a.out_norm ? a.out_norm + (size_t)rhs * a.norm_rhs_stride : nullptr, idx, a.g.stride, out);
@@ -635,14 +642,12 @@ __device__ __forceinline__ Sums3<typename P::real> store_site(const HopArgs& a, 
     site.q[REDUCE == RED_DOT_SELF ? 2 : 0] = nn;
   }
   if constexpr (REDUCE == RED_DOT_AUX) {
-    // (aux, out) = sum conj(aux) out, aux an FP32 field at the output site
-    cplx<float> x[12];
-    load_spinor<PrecS>(x, (const char*)a.aux + (size_t)rhs * a.aux_rhs_bytes, nullptr, idx, a.g.stride);
+    // (aux, out) = sum conj(aux) out
     T re = 0, im = 0;
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      re = fmadd((T)x[k].re, out[k].re, fmadd((T)x[k].im, out[k].im, re));
-      im = fmadd((T)x[k].re, out[k].im, fmadd(-(T)x[k].im, out[k].re, im));
+      re = fmadd((T)aux[k].re, out[k].re, fmadd((T)aux[k].im, out[k].im, re));
+      im = fmadd((T)aux[k].re, out[k].im, fmadd(-(T)aux[k].im, out[k].re, im));
     }
     site.q[0] = re;
     site.q[1] = im;
@@ -660,24 +665,42 @@ __device__ __forceinline__ Sums3<typename P::real> store_site(const HopArgs& a, 
   return site;
 }
 
+// the XPAY operand of one site as it is stored in fp16
+__device__ __forceinline__ HalfSite self_half(const HopArgs& a, int rhs, int idx) {
+  return load_half((const char*)a.self + (size_t)rhs * a.self_rhs_bytes, a.self_norm + (size_t)rhs * a.norm_rhs_stride,
+                   idx, a.g.stride);
+}
+
 template <typename P, int MODE, bool DAG>
 __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, int idx,
                                                    const cplx<typename P::real> (&acc)[12],
                                                    cplx<typename P::real> (&out)[12],
-                                                   cplx<typename P::real> (&self)[12]);
+                                                   cplx<typename P::real> (&self)[12],
+                                                   const HeldSite* held = nullptr);
 
 // The MODE epilogue of one output site: out = a D' psi, T (a D' psi) or T self + a D' psi
 // (+ twist), stored in the output precision; returns the site sums of the REDUCE kind.
 template <typename P, int MODE, bool DAG, int REDUCE>
 __device__ __forceinline__ Sums3<typename P::real> hop_epilogue(const HopArgs& a, int rhs, int idx,
-                                                                const cplx<typename P::real> (&acc)[12]) {
+                                                                const cplx<typename P::real> (&acc)[12],
+                                                                const HeldSite* held = nullptr) {
   static_assert((REDUCE != RED_DOT_SELF && REDUCE != RED_DOT_AUX) || MODE == HOP_XPAY || MODE == HOP_SYM,
                 "the dot-product reductions are fused into the XPAY and SYM epilogues");
   using T = typename P::real;
   cplx<T> out[12];
   cplx<T> self[12];
-  hop_epilogue_value<P, MODE, DAG>(a, rhs, idx, acc, out, self);
-  return store_site<P, REDUCE>(a, rhs, idx, out, self);
+  cplx<float> aux[12];
+  // before the store: a plain load is not moved above it
+  if constexpr (REDUCE == RED_DOT_AUX) {
+    if (held) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) aux[k] = held->aux[k];
+    } else {
+      load_spinor<PrecS>(aux, (const char*)a.aux + (size_t)rhs * a.aux_rhs_bytes, nullptr, idx, a.g.stride);
+    }
+  }
+  hop_epilogue_value<P, MODE, DAG>(a, rhs, idx, acc, out, self, held);
+  return store_site<P, REDUCE>(a, rhs, idx, out, self, aux);
 }
 
 // The output value of the MODE epilogue at one site (self: the XPAY operand, loaded here)
@@ -685,7 +708,8 @@ template <typename P, int MODE, bool DAG>
 __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, int idx,
                                                    const cplx<typename P::real> (&acc)[12],
                                                    cplx<typename P::real> (&out)[12],
-                                                   cplx<typename P::real> (&self)[12]) {
+                                                   cplx<typename P::real> (&self)[12],
+                                                   const HeldSite* held) {
   using T = typename P::real;
   const Geom& g = a.g;
   const T coef = (T)a.a;
@@ -715,8 +739,11 @@ __device__ __forceinline__ void hop_epilogue_value(const HopArgs& a, int rhs, in
       }
     }
   } else {  // HOP_XPAY
-    const char* sp = (const char*)a.self + (size_t)rhs * a.self_rhs_bytes;
-    load_spinor<P>(self, sp, a.self_norm ? a.self_norm + (size_t)rhs * a.norm_rhs_stride : nullptr, idx, g.stride);
+    if constexpr (std::is_same<P, PrecH>::value) {
+      unpack_half(self, held ? held->self : self_half(a, rhs, idx));
+    } else {
+      load_spinor<P>(self, (const char*)a.self + (size_t)rhs * a.self_rhs_bytes, nullptr, idx, g.stride);
+    }
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
       T d[6];

@@ -5,7 +5,9 @@
 // latency-bound (few resident warps, each with one or two hops of loads outstanding): the ring
 // keeps four hops of loads in flight per thread without holding them in registers.  Each thread
 // reads back only the slots it wrote, so no block barrier is needed; a slot is refilled only
-// after the hop that used it has been computed.
+// after the hop that used it has been computed.  The epilogue's operands come through the ring too: as
+// plain loads (the only kind of a field that a predecessor may still be writing, launch.cuh) they
+// stayed behind the last hop's wait.  12 right-hand sides at 32^3 x 64: the solve 385.5 -> 380.7 ms.
 #pragma once
 #include "dslash.cuh"
 
@@ -128,11 +130,48 @@ __device__ __forceinline__ void compute_hop(float2 (&acc)[12], const HopRing<REC
   reconstruct_f2<MU, S>(acc, uh);
 }
 
-// wait for hop H's copies, compute it, and refill its slot with hop H + 4
-template <int RECON, int H, bool DAG, int TX>
+// The epilogue's operands at the site (HOP_XPAY's self; RED_DOT_AUX's aux, half of it at a time) take the
+// slots that hops 4, 5 and 6 leave: their latency passes behind the hops that remain.
+template <int RECON, int TX>
+__device__ __forceinline__ void issue_self(HopRing<RECON, TX>& R, const HopArgs& a, int rhs, int idx) {
+  const int t = threadIdx.x;
+  const uint4* p = reinterpret_cast<const uint4*>((const char*)a.self + (size_t)rhs * a.self_rhs_bytes);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) cp_async16(&R.sp[0][k][t], p + (size_t)k * a.g.stride + idx);
+  cp_async4(&R.nm[0][t], a.self_norm + (size_t)rhs * a.norm_rhs_stride + idx);
+  cp_commit();
+}
+template <int RECON, int TX>
+__device__ __forceinline__ void issue_aux(HopRing<RECON, TX>& R, int half, const HopArgs& a, int rhs, int idx) {
+  const uint4* p = reinterpret_cast<const uint4*>((const char*)a.aux + (size_t)rhs * a.aux_rhs_bytes);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) cp_async16(&R.sp[1 + half][k][threadIdx.x], p + (size_t)(3 * half + k) * a.g.stride + idx);
+  cp_commit();
+}
+template <int RECON, int TX, bool AUX>
+__device__ __forceinline__ HeldSite held_site(const HopRing<RECON, TX>& R) {
+  const int t = threadIdx.x;
+  HeldSite v;
+  v.self.n = R.nm[0][t];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v.self.w[k] = R.sp[0][k][t];
+  if constexpr (AUX) {
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+      const uint4 w = R.sp[1 + k / 3][k % 3][t];
+      v.aux[2 * k] = {__uint_as_float(w.x), __uint_as_float(w.y)};
+      v.aux[2 * k + 1] = {__uint_as_float(w.z), __uint_as_float(w.w)};
+    }
+  }
+  return v;
+}
+
+// wait for hop H's copies (EXTRA groups were issued after hop 7's), compute it, and refill its slot with
+// hop H + 4
+template <int RECON, int H, bool DAG, int TX, int EXTRA>
 __device__ __forceinline__ void ring_step(float2 (&acc)[12], HopRing<RECON, TX>& R, const HopArgs& a,
                                           const HopSites& hs, int idx, const char* in, const float* in_norm) {
-  cp_wait<(H < 4 ? 3 : 7 - H)>();
+  cp_wait<(H < 4 ? 3 : 7 - H + EXTRA)>();
   compute_hop<RECON, H, DAG, TX>(acc, R, hs);
   if constexpr (H + 4 < 8) issue_hop<RECON, TX>(R, H & 3, H + 4, a, hs, idx, in, in_norm);
 }
@@ -157,18 +196,28 @@ __global__ void __launch_bounds__(TX, MINB) hop_kernel_async(const HopArgs a) {
     float2 acc[12];
 #pragma unroll
     for (int k = 0; k < 12; ++k) acc[k] = make_float2(0.f, 0.f);
-    ring_step<RECON, 0, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 1, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 2, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 3, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 4, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 5, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 6, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
-    ring_step<RECON, 7, DAG, TX>(acc, R, a, hs, idx, in, in_norm);
+    constexpr bool kSelf = MODE == HOP_XPAY, kAux = REDUCE == RED_DOT_AUX;
+    static_assert(MODE != HOP_SYM && (kSelf || !kAux), "epilogue operands");
+    ring_step<RECON, 0, DAG, TX, 0>(acc, R, a, hs, idx, in, in_norm);
+    ring_step<RECON, 1, DAG, TX, 0>(acc, R, a, hs, idx, in, in_norm);
+    ring_step<RECON, 2, DAG, TX, 0>(acc, R, a, hs, idx, in, in_norm);
+    ring_step<RECON, 3, DAG, TX, 0>(acc, R, a, hs, idx, in, in_norm);
+    ring_step<RECON, 4, DAG, TX, 0>(acc, R, a, hs, idx, in, in_norm);
+    if constexpr (kSelf) issue_self<RECON, TX>(R, a, rhs, idx);
+    ring_step<RECON, 5, DAG, TX, kSelf>(acc, R, a, hs, idx, in, in_norm);
+    if constexpr (kAux) issue_aux<RECON, TX>(R, 0, a, rhs, idx);
+    ring_step<RECON, 6, DAG, TX, kSelf + kAux>(acc, R, a, hs, idx, in, in_norm);
+    if constexpr (kAux) issue_aux<RECON, TX>(R, 1, a, rhs, idx);
+    ring_step<RECON, 7, DAG, TX, kSelf + 2 * kAux>(acc, R, a, hs, idx, in, in_norm);
+    HeldSite held;
+    if constexpr (kSelf) {
+      cp_wait<0>();
+      held = held_site<RECON, TX, kAux>(R);
+    }
     cplx<float> out[12];
 #pragma unroll
     for (int k = 0; k < 12; ++k) out[k] = {acc[k].x, acc[k].y};
-    local = hop_epilogue<PrecH, MODE, DAG, REDUCE>(a, rhs, idx, out);
+    local = hop_epilogue<PrecH, MODE, DAG, REDUCE>(a, rhs, idx, out, kSelf ? &held : nullptr);
   }
   if constexpr (REDUCE != RED_NONE) block_sums_1rhs<red_count<REDUCE>(), TX>(a, local, rhs, sblock, (g.Vh + TX - 1) / TX);
 }

@@ -267,20 +267,34 @@ __device__ __forceinline__ void load_spinor<PrecS>(cplx<float> (&s)[12], const v
     s[2 * k + 1] = {v.z, v.w};
   }
 }
-template <>
-__device__ __forceinline__ void load_spinor<PrecH>(cplx<float> (&s)[12], const void* base, const float* norm, int idx,
-                                                   int stride) {
+// one fp16 site as stored
+struct HalfSite {
+  uint4 w[3];
+  float n;
+};
+__device__ __forceinline__ HalfSite load_half(const void* base, const float* norm, int idx, int stride) {
   const uint4* p = reinterpret_cast<const uint4*>(base);
-  float n = ldw(norm + idx);
+  HalfSite v;
+  v.n = ldw(norm + idx);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v.w[k] = ldw(p + (size_t)k * stride + idx);
+  return v;
+}
+__device__ __forceinline__ void unpack_half(cplx<float> (&s)[12], const HalfSite& v) {
+  const float n = v.n;
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    uint4 v = ldw(p + (size_t)k * stride + idx);
-    float2 a = h2f(v.x), b = h2f(v.y), c = h2f(v.z), d = h2f(v.w);
+    const float2 a = h2f(v.w[k].x), b = h2f(v.w[k].y), c = h2f(v.w[k].z), d = h2f(v.w[k].w);
     s[4 * k + 0] = {a.x * n, a.y * n};
     s[4 * k + 1] = {b.x * n, b.y * n};
     s[4 * k + 2] = {c.x * n, c.y * n};
     s[4 * k + 3] = {d.x * n, d.y * n};
   }
+}
+template <>
+__device__ __forceinline__ void load_spinor<PrecH>(cplx<float> (&s)[12], const void* base, const float* norm, int idx,
+                                                   int stride) {
+  unpack_half(s, load_half(base, norm, idx, stride));
 }
 
 // A double-float kernel reads its spinor operands from their split copies (made once per launch by
