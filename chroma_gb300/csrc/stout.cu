@@ -227,6 +227,7 @@ extern "C" int gbc_stout_smear(const gbc_geom* geom, int n_steps, double rho, co
   if (cudaMalloc(&buf[0], bytes) != cudaSuccess || cudaMalloc(&buf[1], bytes) != cudaSuccess ||
       cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
     rc = GBC_ERR_CUDA;
+    (void)cudaGetLastError();  // reported here: the thread's next call must not find it
   } else {
     try {
       touch.populate({{links_out, bytes}}, nullptr, PageTouch::kThreads);
