@@ -624,12 +624,12 @@ struct HeldSite {
 };
 
 // Store one output site in the output precision and return its site sums of the REDUCE kind
-// (self: the XPAY operand, for RED_DOT_SELF; aux: the FP32 field at the site, for RED_DOT_AUX).
+// (self: the XPAY operand, for RED_DOT_SELF).
 template <typename P, int REDUCE>
 __device__ __forceinline__ Sums3<typename P::real> store_site(const HopArgs& a, int rhs, int idx,
                                                               const cplx<typename P::real> (&out)[12],
                                                               const cplx<typename P::real> (&self)[12],
-                                                              const cplx<float> (&aux)[12]) {
+                                                              const HeldSite* held) {
   using T = typename P::real;
   char* op = (char*)a.out + (size_t)rhs * a.out_rhs_bytes;
   store_spinor<P>(op, a.out_norm ? a.out_norm + (size_t)rhs * a.norm_rhs_stride : nullptr, idx, a.g.stride, out);
@@ -642,12 +642,19 @@ __device__ __forceinline__ Sums3<typename P::real> store_site(const HopArgs& a, 
     site.q[REDUCE == RED_DOT_SELF ? 2 : 0] = nn;
   }
   if constexpr (REDUCE == RED_DOT_AUX) {
-    // (aux, out) = sum conj(aux) out
+    // (aux, out) = sum conj(aux) out, aux an FP32 field at the output site
+    cplx<float> x[12];
+    if (held) {
+#pragma unroll
+      for (int k = 0; k < 12; ++k) x[k] = held->aux[k];
+    } else {
+      load_spinor<PrecS>(x, (const char*)a.aux + (size_t)rhs * a.aux_rhs_bytes, nullptr, idx, a.g.stride);
+    }
     T re = 0, im = 0;
 #pragma unroll
     for (int k = 0; k < 12; ++k) {
-      re = fmadd((T)aux[k].re, out[k].re, fmadd((T)aux[k].im, out[k].im, re));
-      im = fmadd((T)aux[k].re, out[k].im, fmadd(-(T)aux[k].im, out[k].re, im));
+      re = fmadd((T)x[k].re, out[k].re, fmadd((T)x[k].im, out[k].im, re));
+      im = fmadd((T)x[k].re, out[k].im, fmadd(-(T)x[k].im, out[k].re, im));
     }
     site.q[0] = re;
     site.q[1] = im;
@@ -689,18 +696,8 @@ __device__ __forceinline__ Sums3<typename P::real> hop_epilogue(const HopArgs& a
   using T = typename P::real;
   cplx<T> out[12];
   cplx<T> self[12];
-  cplx<float> aux[12];
-  // before the store: a plain load is not moved above it
-  if constexpr (REDUCE == RED_DOT_AUX) {
-    if (held) {
-#pragma unroll
-      for (int k = 0; k < 12; ++k) aux[k] = held->aux[k];
-    } else {
-      load_spinor<PrecS>(aux, (const char*)a.aux + (size_t)rhs * a.aux_rhs_bytes, nullptr, idx, a.g.stride);
-    }
-  }
   hop_epilogue_value<P, MODE, DAG>(a, rhs, idx, acc, out, self, held);
-  return store_site<P, REDUCE>(a, rhs, idx, out, self, aux);
+  return store_site<P, REDUCE>(a, rhs, idx, out, self, held);
 }
 
 // The output value of the MODE epilogue at one site (self: the XPAY operand, loaded here)
