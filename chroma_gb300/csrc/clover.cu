@@ -106,7 +106,7 @@ __device__ __forceinline__ M plane_field(const double2* u, long s, long up_m, lo
 // A block builds 32 sites: warp k computes the field strength of plane k (lane = site), then warps 0
 // and 1 assemble, store and invert chirality blocks 0 and 1; the block's sums of log|d| per parity and
 // of the even sites' negative pivots.  Bound by the FP64 pipe: 1080 FP64 instructions per plane and site
-// and about 700 per chirality block.  One thread per site held six field strengths and both blocks at
+// and about 1070 per chirality block.  One thread per site held six field strengths and both blocks at
 // once and spilled them.
 __global__ void __launch_bounds__(6 * kBuildSites, 2) clover_build_kernel(Dims D, const double2* canon, CloverCoeffs cc,
                                                                        double* clov, double* inv, int inv_parity, long V,

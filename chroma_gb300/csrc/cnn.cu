@@ -232,15 +232,15 @@ constexpr int kTmemCols = 32;  // tensor-memory columns allocated per block (>= 
 // right-hand side).  Against one task per (site, direction, channel) with the transports in shared
 // memory, this mapping reads whole 512-byte rows, keeps each transport in registers for every
 // channel and right-hand side and writes 16 bytes per shared-memory store.  A 12 -> 12 layer at
-// 16^3 x 32: 1772 -> 492 us for 12 right-hand sides, 217 -> 60 us for one (kernel time, cold L2).
+// 16^3 x 32: 1772 -> 505 us for 12 right-hand sides, 217 -> 56 us for one (kernel time, cold L2).
 // IN_ODD: only the self term of odd sites and the hops of even sites are non-zero; the others'
 // columns of G are zeroed, and odd sites need only the K steps that cover the self term.
 // A block walks its tiles: weights, tensor memory and barrier are set up once, and warps 3..8 gather
-// the next tile while warps 0..2 still store this one.
+// the next tile while warps 0..2 still store this one (one right-hand side 60 -> 56 us; twelve, which
+// fill the chip with a block per tile too, 492 -> 505).
 // Every thread waits for the MMA on its own clock, so a warp votes on the outcome: it uses its
 // accumulator rows (tcgen05.ld needs the whole warp) or counts one error (its network's, read by the
-// host) and stores nothing.  Warp
-// `quit` (-1: none) gives up its first wait at once, for tests of that path.
+// host) and stores nothing.  Warp `quit` (-1: none) gives up its first wait at once, for tests of that path.
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(CT, 3) layer_kernel(Geom g, int V, int tiles, int total, int batch, int per, int flags,
                                                       const float2* __restrict__ links, const float4* __restrict__ hin,

@@ -1,7 +1,7 @@
 // FP64 hopping term with fused clover epilogues, the 8 hops of a site split over 8 threads.
 //
 // What bounds it: the FP64 pipe.  GB300 retires about two FP64 lane operations per SM and clock, so
-// a 32-site tile of A_ee^-1 D_eo (1128 FP64 instructions per site) keeps one SM busy for about 9 us
+// a 32-site tile of A_ee^-1 D_eo (1136 FP64 instructions per site) keeps one SM busy for about 9 us
 // however many warps it has, and a lattice is fast only when its sites are spread evenly over all
 // 152 SMs.  One thread per site in blocks of 128 (hop_kernel) leaves a 4096-site checkerboard on 32
 // SMs; splitting the hops makes blocks of 8 to 32 sites that still have 2 to 8 warps.

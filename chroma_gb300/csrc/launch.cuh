@@ -3,7 +3,7 @@
 // predecessor's completion and memory.  Its blocks then fill the places that the last wave leaves.
 //
 // A kernel launched this way calls pdl_begin() before it touches memory, and reads what other kernels
-// write with ordinary loads (ldw): the read-only path is for data that no kernel in flight writes (links,
+// write with ordinary loads (ldw) or cp.async: the read-only path is for data that no kernel in flight writes (links,
 // clover: packed before a host synchronisation).
 #pragma once
 #include <cuda_runtime.h>

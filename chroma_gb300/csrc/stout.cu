@@ -14,7 +14,7 @@
 // links through L1/L2 (each link is read by up to 18 staples).  Links of directions that are not
 // smeared are copied.
 // What bounds it: the FP64 pipe (about two lane operations per SM and clock), with 1296 FP64
-// instructions per link in the staples and about 500 in the rest.  So each staple's second product
+// instructions per link in the staples and about 480 in the rest.  So each staple's second product
 // accumulates into the sum, Q and Q^2 are kept as the 3 real and 3 complex numbers of a Hermitian
 // matrix, and the Taylor coefficients are scalar recursions (8 instructions a term).
 #include <cuda_runtime.h>
